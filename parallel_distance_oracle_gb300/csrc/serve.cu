@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(256) serve_query_kernel(const ServeRun *__rest
                                                           const uint32_t *__restrict__ qb,
                                                           unsigned char *__restrict__ out)
 {
+    __shared__ QueryScratch qs[8];
     const int lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -77,10 +78,10 @@ __global__ void __launch_bounds__(256) serve_query_kernel(const ServeRun *__rest
         const ServeRun &run = runs[r];
         const uint64_t i = p - run.start;
         if (run.weighted) {
-            const int16_t d = query_w_pair(run.v, qa[p], qb[p], lane, bytes);
+            const int16_t d = query_w_pair(run.v, qa[p], qb[p], lane, qs[threadIdx.x >> 5], bytes);
             if (lane == 0) reinterpret_cast<int16_t *>(out + run.out_off)[i] = d;
         } else {
-            const uint8_t d = query_unw_pair(run.v, qa[p], qb[p], lane, bytes);
+            const uint8_t d = query_unw_pair(run.v, qa[p], qb[p], lane, qs[threadIdx.x >> 5], bytes);
             if (lane == 0) out[run.out_off + i] = d;
         }
     }
