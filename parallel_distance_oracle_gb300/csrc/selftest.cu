@@ -18,7 +18,8 @@ namespace {
 __global__ void barrier_selftest_kernel(GridBar *bar, uint32_t *status, uint32_t absent,
                                         unsigned long long timeout_ns, uint32_t *returned)
 {
-    if (blockIdx.x != absent) grid_barrier(bar, status, timeout_ns);
+    GridSync sync(bar, status);
+    if (blockIdx.x != absent) sync.wait(timeout_ns);
     __syncthreads();
     if (threadIdx.x == 0) atomicAdd(returned, 1u);
 }

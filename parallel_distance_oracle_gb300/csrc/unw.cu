@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, L
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+    GridSync sync(&c->bar, &c->status);
     // the loop state lives in registers; every block derives the same
     // transitions from the same post-barrier counters
     uint32_t phase = vload(&c->phase), b = vload(&c->b), iter = vload(&c->iter), L = vload(&c->lid) + 1;
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, L
                 c->tq[(L + 2) % 3] = 0;
                 c->hq[(L + 2) % 3] = 0;
             }
-            if (!grid_barrier(&c->bar, &c->status)) return;
+            if (!sync.wait()) return;
             if (vload(&c->retry_cnt)) {
                 if (leader) {
                     c->phase = PH_ROOT_RETRY;
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, L
             c->tq[(L + 2) % 3] = 0;
             c->hq[(L + 2) % 3] = 0;
         }
-        if (!grid_barrier(&c->bar, &c->status)) return;
+        if (!sync.wait()) return;
         if (vload(&c->retry_cnt)) {
             if (leader) {
                 c->phase = PH_PULL_RETRY;
@@ -459,7 +460,6 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
             PADO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, PULL_THREADS, smem));
             PADO_CHECK(per_sm >= 1, PADO_E_CUDA, "labeling loop kernel cannot be resident");
             const unsigned grid = (unsigned)(sms * std::min(per_sm, 4));  // compiled for 4 blocks/SM
-            PADO_CHECK(grid <= BAR_GROUP * BAR_MAX_GROUPS, PADO_E_CUDA, "grid larger than the barrier supports");
             LoopCtl h{};
             LoopCtl *cp_ = ctl.p;
             for (int launch = 0;; ++launch) {
@@ -491,6 +491,7 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
                     h.hcnt[cur] = 0;
                 }
                 for (int x = 0; x < 3; ++x) h.tq[x] = h.hq[x] = 0;  // the re-run level claims from zero
+                h.bar = GridBar{};  // a launch starts its barriers from zero
                 h.retry_cnt = 0;
                 h.status = 0;
                 h.exit_code = EX_RUNNING;

@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) many_loop_kernel(UnwDev d, Ma
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+    GridSync sync(&c->bar, &c->status);
     for (;;) {
         const uint32_t phase = vload(&c->phase);
         if (phase == MP_DONE) return;
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) many_loop_kernel(UnwDev d, Ma
             c->tq[(L + 2) % 3] = 0;
             c->hq[(L + 2) % 3] = 0;
         }
-        if (!grid_barrier(&c->bar, &c->status)) return;
+        if (!sync.wait()) return;
         if (vload(&c->rretry_cnt) || vload(&c->tretry_cnt)) {
             if (leader) {
                 c->phase = MP_RETRY;
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) many_loop_kernel(UnwDev d, Ma
             c->zq_cnt[cp] = 0;
             c->phase = MP_STEP;
         }
-        if (!grid_barrier(&c->bar, &c->status)) return;
+        if (!sync.wait()) return;
         if (vload(&c->status) & ST_LEVEL_OVERFLOW) {
             if (leader) {
                 c->phase = MP_DONE;
@@ -450,6 +451,7 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
                 h.tcnt[cur] = h.tretry_cnt;
                 h.hcnt[cur] = 0;
                 for (int x = 0; x < 3; ++x) h.tq[x] = h.hq[x] = 0;  // the re-run step claims from zero
+                h.bar = GridBar{};  // a launch starts its barriers from zero
                 h.rretry_cnt = 0;
                 h.tretry_cnt = 0;
                 h.status = 0;

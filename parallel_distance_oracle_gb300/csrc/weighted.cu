@@ -774,6 +774,7 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
 {
     extern __shared__ __align__(16) unsigned char wsm[];
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+    GridSync sync(&c->bar, &c->status);
     uint32_t phase = vload(&c->phase), b = vload(&c->b), lid = vload(&c->lid);
     uint32_t rounds = vload(&c->rounds), levels = vload(&c->levels);
     auto save = [&](uint32_t ph, uint32_t ex) {
@@ -805,7 +806,7 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
                 c->tq[(lid0 + 2) % 3] = 0;
                 d.log_top[(lid0 + 1) & 1] = 0;     // the first round's log
             }
-            if (!grid_barrier(&c->bar, &c->status)) return;
+            if (!sync.wait()) return;
             lid = lid0;
             rounds = 0;
             phase = WP_ROUND;
@@ -823,7 +824,7 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
                 if (b == 0) {
                     // check (2) reads the batch's temporary tables as of the round start
                     w_snap_phase(d, nr);
-                    if (!grid_barrier(&c->bar, &c->status)) return;
+                    if (!sync.wait()) return;
                 }
             }
             w_pull_phase(d, bf.tails[tp], vload(&c->tails_cnt[tp]), s, b, lid_cur, nullptr, nullptr, bf.news[b & 1],
@@ -834,7 +835,7 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
                 c->tq[(lid_cur + 2) % 3] = 0;
                 d.log_top[(lid_cur + 1) & 1] = 0;     // the next round's log, last read by this pull
             }
-            if (!grid_barrier(&c->bar, &c->status)) return;
+            if (!sync.wait()) return;
             if (vload(&c->retry_cnt)) {
                 save(WP_PULL_RETRY, WX_NEED_LOG);
                 return;
@@ -860,10 +861,10 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
                     // their chunks after the first are spread over the grid,
                     // and the commit follows once every filter is done
                     w_filter_phase(d, bf.news[nb], nn, s, bf.heavy, &c->heavy_cnt);
-                    if (!grid_barrier(&c->bar, &c->status)) return;
+                    if (!sync.wait()) return;
                     w_filter_heavy_phase(d, bf.heavy, vload(&c->heavy_cnt), s);
                     w_buf_reset_phase(d, s, nr);
-                    if (!grid_barrier(&c->bar, &c->status)) return;
+                    if (!sync.wait()) return;
                     w_commit_phase(d, bf.news[nb], nn, s, bf.retry, &c->retry_cnt);
                 } else {
                     // filter and commit each vertex in one go; the roots'
@@ -875,7 +876,7 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
             } else {
                 w_commit_phase(d, bf.rr, vload(&c->rr_cnt), s, bf.retry, &c->retry_cnt);
             }
-            if (!grid_barrier(&c->bar, &c->status)) return;
+            if (!sync.wait()) return;
             if (vload(&c->retry_cnt)) {
                 save(WP_COMMIT_RETRY, WX_NEED_POOL);
                 return;
@@ -1036,7 +1037,6 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
             PADO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, WPULL_WARPS * 32, pull_smem));
             PADO_CHECK(per_sm >= 1, PADO_E_CUDA, "weighted labeling loop kernel cannot be resident");
             const unsigned grid = (unsigned)(sms * std::min(per_sm, 8));
-            PADO_CHECK(grid <= BAR_GROUP * BAR_MAX_GROUPS, PADO_E_CUDA, "grid larger than the barrier supports");
             WLoopCtl h{};
             WLoopCtl *cptr = ctl.p;
             for (int launch = 0;; ++launch) {
@@ -1071,6 +1071,7 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
                     PADO_CUDA(cudaMemcpyAsync(rr.p, retry.p, h.retry_cnt * 4ull, cudaMemcpyDeviceToDevice, s));
                     h.rr_cnt = h.retry_cnt;
                 }
+                h.bar = GridBar{};  // a launch starts its barriers from zero
                 h.retry_cnt = 0;
                 h.status = 0;
                 h.exit_code = WX_RUNNING;
