@@ -58,66 +58,113 @@ constexpr uint32_t TEXT_CHUNK = 16;              // bytes per thread when locati
 
 // ---- scan -------------------------------------------------------------------
 
-// Exclusive scan of a[0, L) in blocks of 1024: per-block scan, block totals in sums.
-__global__ void __launch_bounds__(1024) scan_block_kernel(uint32_t *a, uint64_t L, uint32_t *sums)
+// Exclusive scan of a[0, L) in blocks of SCAN_TILE: per-block scan, block
+// totals in sums, the totals scanned by one block, and added back.  Bound by
+// memory: 16 bytes per access, 8 entries per thread, shuffles within a warp
+// and two barriers per block.
+constexpr int SCAN_THREADS = 512;
+constexpr uint32_t SCAN_TILE = SCAN_THREADS * 8;
+
+// Exclusive prefix of x over the block; *total receives the block's sum.
+template <int T>
+__device__ __forceinline__ uint32_t block_prefix(uint32_t x, uint32_t *total)
 {
-    __shared__ uint32_t s[1024];
-    const uint64_t i = (uint64_t)blockIdx.x * 1024 + threadIdx.x;
-    const uint32_t x = i < L ? a[i] : 0u;
-    s[threadIdx.x] = x;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const uint32_t y = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0u;
-        __syncthreads();
-        s[threadIdx.x] += y;
-        __syncthreads();
+    __shared__ uint32_t wsum[T / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t inc = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULLW, inc, o);
+        if (lane >= o) inc += y;
     }
-    if (i < L) a[i] = s[threadIdx.x] - x;
-    if (threadIdx.x == 1023) sums[blockIdx.x] = s[1023];
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    uint32_t v = lane < T / 32 ? wsum[lane] : 0u;
+#pragma unroll
+    for (int o = 1; o < T / 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULLW, v, o);
+        if (lane >= o) v += y;
+    }
+    const uint32_t before = __shfl_sync(FULLW, v, w > 0 ? w - 1 : 0);
+    *total = __shfl_sync(FULLW, v, T / 32 - 1);
+    __syncthreads();  // wsum may be reused
+    return (w > 0 ? before : 0u) + inc - x;
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) scan_block_kernel(uint32_t *a, uint64_t L, uint32_t *sums)
+{
+    const uint64_t i = ((uint64_t)blockIdx.x * SCAN_THREADS + threadIdx.x) * 8;
+    uint32_t x[8];
+    if (i + 8 <= L) {
+        *reinterpret_cast<uint4 *>(x) = *reinterpret_cast<const uint4 *>(a + i);
+        *reinterpret_cast<uint4 *>(x + 4) = *reinterpret_cast<const uint4 *>(a + i + 4);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = i + q < L ? a[i + q] : 0u;
+    }
+    uint32_t sum = 0, total;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const uint32_t y = x[q];
+        x[q] = sum;
+        sum += y;
+    }
+    const uint32_t pre = block_prefix<SCAN_THREADS>(sum, &total);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) x[q] += pre;
+    if (i + 8 <= L) {
+        *reinterpret_cast<uint4 *>(a + i) = *reinterpret_cast<const uint4 *>(x);
+        *reinterpret_cast<uint4 *>(a + i + 4) = *reinterpret_cast<const uint4 *>(x + 4);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (i + q < L) a[i + q] = x[q];
+    }
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
 // One block: exclusive scan of the nb block totals, 1024 at a time.
 __global__ void __launch_bounds__(1024) scan_sums_kernel(uint32_t *sums, uint32_t nb)
 {
-    __shared__ uint32_t s[1024];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
+    uint32_t carry = 0;
     for (uint32_t c0 = 0; c0 < nb; c0 += 1024) {
         const uint32_t i = c0 + threadIdx.x;
-        const uint32_t x = i < nb ? sums[i] : 0u;
-        s[threadIdx.x] = x;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            const uint32_t y = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0u;
-            __syncthreads();
-            s[threadIdx.x] += y;
-            __syncthreads();
-        }
-        if (i < nb) sums[i] = carry + s[threadIdx.x] - x;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += s[1023];
-        __syncthreads();
+        uint32_t total;
+        const uint32_t pre = block_prefix<1024>(i < nb ? sums[i] : 0u, &total);
+        if (i < nb) sums[i] = carry + pre;
+        carry += total;
     }
 }
 
-__global__ void __launch_bounds__(1024) scan_add_kernel(uint32_t *a, uint64_t L, const uint32_t *sums)
+__global__ void __launch_bounds__(SCAN_THREADS) scan_add_kernel(uint32_t *a, uint64_t L, const uint32_t *sums)
 {
-    const uint64_t i = (uint64_t)blockIdx.x * 1024 + threadIdx.x;
-    if (i < L) a[i] += sums[blockIdx.x];
+    const uint64_t i = ((uint64_t)blockIdx.x * SCAN_THREADS + threadIdx.x) * 8;
+    const uint32_t s = sums[blockIdx.x];
+    if (i + 8 <= L) {
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {
+            uint4 x = *reinterpret_cast<const uint4 *>(a + i + q);
+            x.x += s, x.y += s, x.z += s, x.w += s;
+            *reinterpret_cast<uint4 *>(a + i + q) = x;
+        }
+    } else {
+        for (uint64_t j = i; j < L; ++j) a[j] += s;
+    }
 }
 
-uint64_t scan_sums_needed(uint64_t L) { return std::max<uint64_t>((L + 1023) / 1024, 1); }
+uint64_t scan_sums_needed(uint64_t L) { return std::max<uint64_t>((L + SCAN_TILE - 1) / SCAN_TILE, 1); }
 
-// In place, stream-ordered; `sums` holds scan_sums_needed(L) entries; the
-// caller keeps the total below 2^32.
+// In place, stream-ordered; `a` is the start of an allocation (16-byte
+// accesses), `sums` holds scan_sums_needed(L) entries; the caller keeps the
+// total below 2^32.
 void exclusive_scan(uint32_t *a, uint64_t L, uint32_t *sums, cudaStream_t s)
 {
     if (L == 0) return;
-    const uint32_t nb = (uint32_t)((L + 1023) / 1024);
-    PADO_LAUNCH("scan_block_kernel", s, scan_block_kernel<<<nb, 1024, 0, s>>>(a, L, sums));
+    const uint32_t nb = (uint32_t)((L + SCAN_TILE - 1) / SCAN_TILE);
+    PADO_LAUNCH("scan_block_kernel", s, scan_block_kernel<<<nb, SCAN_THREADS, 0, s>>>(a, L, sums));
+    if (nb == 1) return;  // one block's prefixes are the scan
     PADO_LAUNCH("scan_sums_kernel", s, scan_sums_kernel<<<1, 1024, 0, s>>>(sums, nb));
-    PADO_LAUNCH("scan_add_kernel", s, scan_add_kernel<<<nb, 1024, 0, s>>>(a, L, sums));
+    PADO_LAUNCH("scan_add_kernel", s, scan_add_kernel<<<nb, SCAN_THREADS, 0, s>>>(a, L, sums));
 }
 
 // Same with its own block-sum buffer; completes before returning.
@@ -193,51 +240,81 @@ struct PBuf {
 
 // ---- radix sort -------------------------------------------------------------
 
-// counts[d * ntiles + tile] = keys of `tile` whose digit at `shift` is d.
+// The keys are split into `gridDim.x` runs of `per` whole tiles, a block
+// each, in all three kernels of a pass.
+
+// counts[d * blocks + block] = keys of the block's run whose digit at `shift` is d.
 __global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const uint64_t *keys, uint64_t L, uint32_t shift,
-                                                             uint32_t ntiles, uint32_t *counts)
+                                                             uint32_t per, uint32_t *counts)
 {
     __shared__ uint32_t h[256];
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        h[threadIdx.x] = 0;
-        __syncthreads();
-        const uint64_t t0 = (uint64_t)tile * RS_TILE, t1 = min(L, t0 + RS_TILE);
-        for (uint64_t i = t0 + threadIdx.x; i < t1; i += RS_THREADS)
-            atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
-        __syncthreads();
-        counts[(uint64_t)threadIdx.x * ntiles + tile] = h[threadIdx.x];
-        __syncthreads();
-    }
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t t0 = (uint64_t)blockIdx.x * per * RS_TILE, t1 = min(L, t0 + (uint64_t)per * RS_TILE);
+#pragma unroll 8
+    for (uint64_t i = t0 + threadIdx.x; i < t1; i += RS_THREADS) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
+    __syncthreads();
+    counts[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
 }
 
-// Stable scatter of one digit.  Warp w owns keys [512 w, 512 w + 512) of the
+// One block per digit: its counts become their exclusive prefix over the runs,
+// totals[d] their sum.
+__global__ void __launch_bounds__(RS_THREADS) rs_scan_kernel(uint32_t *counts, uint32_t nruns, uint32_t *totals)
+{
+    uint32_t *c = counts + (uint64_t)blockIdx.x * nruns;
+    uint32_t carry = 0;
+    for (uint32_t c0 = 0; c0 < nruns; c0 += RS_THREADS) {
+        const uint32_t i = c0 + threadIdx.x;
+        uint32_t total;
+        const uint32_t pre = block_prefix<RS_THREADS>(i < nruns ? c[i] : 0u, &total);
+        if (i < nruns) c[i] = carry + pre;
+        carry += total;
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+// Where the last pass of an entry sort puts its result: the adjacency and
+// weights read out of the keys (see the file comment) instead of the keys.
+struct EntryOut {
+    uint32_t bits = 0;
+    uint32_t *adj = nullptr;
+    uint8_t *w = nullptr;
+};
+
+// Stable scatter of one digit.  Warp w owns keys [512 w, 512 w + 512) of a
 // tile, 32 per round; a key's place among the tile's keys with its digit is
 // (keys of lower warps) + (keys of earlier rounds of its warp) + (lower lanes
 // of its round), which is its input order.  A thread's 16 keys are loaded
-// before any ranking so that their loads are in flight together.
+// before any ranking so that their loads are in flight together.  A block
+// takes its run tile by tile and moves each digit's position on as it goes, so
+// the pass needs counts per run only, not per tile.
+template <bool ENTRIES>
 __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_t *in, uint64_t *out, uint64_t L,
-                                                                uint32_t shift, uint32_t ntiles,
-                                                                const uint32_t *offsets)
+                                                                uint32_t shift, uint32_t per,
+                                                                const uint32_t *counts, const uint32_t *totals,
+                                                                EntryOut eo)
 {
     constexpr int NW = RS_THREADS / 32;
     __shared__ uint64_t sk[RS_TILE];      // the tile, reordered by digit
     __shared__ uint16_t slr[RS_TILE];     // rank of key i among its warp's keys with its digit
     __shared__ uint16_t wcnt[NW][256];    // per warp and digit: count, then prefix over warps
     __shared__ uint32_t dstart[256];      // first slot of each digit in the reordered tile
-    __shared__ uint32_t gbase[256];       // global position of each digit's run
-    __shared__ uint32_t wsum[NW];
+    __shared__ uint32_t gbase[256];       // global position of slot 0 as each digit's run sees it
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint64_t t0 = (uint64_t)tile * RS_TILE;
-        const uint32_t cnt = (uint32_t)min(L - t0, (uint64_t)RS_TILE);
+    uint32_t unused;
+    // thread d: global position of the run's next key with digit d
+    uint32_t pos = block_prefix<RS_THREADS>(totals[threadIdx.x], &unused) +
+                   counts[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x];
+    const uint64_t run0 = (uint64_t)blockIdx.x * per * RS_TILE, run1 = min(L, run0 + (uint64_t)per * RS_TILE);
+    for (uint64_t t0 = run0; t0 < run1; t0 += RS_TILE) {
+        const uint32_t cnt = (uint32_t)min(run1 - t0, (uint64_t)RS_TILE);
         const uint32_t i0 = wl * (RS_PER * 32) + lane;
         uint64_t key[RS_PER];
 #pragma unroll
         for (int r = 0; r < RS_PER; ++r) key[r] = i0 + r * 32 < cnt ? in[t0 + i0 + r * 32] : 0ull;
 #pragma unroll
         for (int w = 0; w < NW; ++w) wcnt[w][threadIdx.x] = 0;
-        gbase[threadIdx.x] = offsets[(uint64_t)threadIdx.x * ntiles + tile];
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < RS_PER; ++r) {
@@ -259,19 +336,10 @@ __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_
             wcnt[w][threadIdx.x] = (uint16_t)tot;
             tot += c;
         }
-        // exclusive scan of the 256 totals -> dstart
-        uint32_t inc = tot;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULLW, inc, o);
-            if (lane >= o) inc += y;
-        }
-        if (lane == 31) wsum[wl] = inc;
-        __syncthreads();
-        uint32_t wpre = 0;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) wpre += w < wl ? wsum[w] : 0u;
-        dstart[threadIdx.x] = wpre + inc - tot;
+        const uint32_t ds = block_prefix<RS_THREADS>(tot, &unused);
+        dstart[threadIdx.x] = ds;
+        gbase[threadIdx.x] = pos - ds;
+        pos += tot;
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < RS_PER; ++r) {
@@ -282,46 +350,69 @@ __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_
             }
         }
         __syncthreads();
+        const uint64_t dmask = (1ull << eo.bits) - 1;
         for (uint32_t p = threadIdx.x; p < cnt; p += RS_THREADS) {
             const uint64_t k = sk[p];
-            const uint32_t dig = (uint32_t)((k >> shift) & 255u);
-            out[gbase[dig] + (p - dstart[dig])] = k;
+            const uint32_t o = gbase[(uint32_t)((k >> shift) & 255u)] + p;
+            if (ENTRIES) {
+                eo.adj[o] = (uint32_t)(dmask - ((k >> 8) & dmask));
+                if (eo.w) eo.w[o] = (uint8_t)(255u - (uint32_t)(k & 255u));
+            } else {
+                out[o] = k;
+            }
         }
         __syncthreads();
     }
 }
 
-uint64_t sort_tiles(uint64_t L) { return std::max<uint64_t>((L + RS_TILE - 1) / RS_TILE, 1); }
+// Runs of a sort of L keys: one per resident block of the scatter, or one per
+// tile where there are fewer.
+constexpr uint32_t RS_MAX_RUNS = 152u * 4u;
+
+uint32_t sort_runs(uint64_t L, uint32_t *per)
+{
+    const uint64_t tiles = (L + RS_TILE - 1) / RS_TILE;
+    *per = (uint32_t)std::max<uint64_t>((tiles + RS_MAX_RUNS - 1) / RS_MAX_RUNS, 1);
+    return (uint32_t)std::max<uint64_t>((tiles + *per - 1) / *per, 1);
+}
 
 // Scratch of a radix sort of up to L keys.
 struct SortSpace {
     PBuf<uint64_t> tmp;
-    PBuf<uint32_t> counts, sums;
+    PBuf<uint32_t> counts, totals;
     SortSpace(uint64_t L, cudaStream_t s)
-        : tmp(std::max<uint64_t>(L, 1), s), counts(256 * sort_tiles(L), s),
-          sums(scan_sums_needed(256 * sort_tiles(L)), s)
+        : tmp(std::max<uint64_t>(L, 1), s),
+          counts(256 * std::min<uint64_t>((L + RS_TILE - 1) / RS_TILE + 1, RS_MAX_RUNS), s), totals(256, s)
     {
     }
 };
 
 // Sorts keys[0, L) ascending on bits [lo, hi), stably, stream-ordered;
-// returns the buffer holding the result (`keys` or ws.tmp).  The dedupe and
+// returns the buffer holding the result (`keys` or ws.tmp; nothing useful with
+// `eo`, whose arrays the last pass writes instead).  The dedupe and
 // vertex-order sorts (`aux`) are profiled under their own names, so that the
 // entry sort's launches all process the same 2m keys.
 uint64_t *radix_sort(uint64_t *keys, uint64_t L, uint32_t lo, uint32_t hi, SortSpace &ws, cudaStream_t s,
-                     bool aux = false)
+                     bool aux = false, const EntryOut *eo = nullptr)
 {
-    if (L < 2 || lo >= hi) return keys;
+    if ((L < 2 && !eo) || lo >= hi) return keys;
     PADO_CHECK(ws.tmp.n >= L, PADO_E_ARG, "sort scratch too small");
-    const uint32_t ntiles = (uint32_t)((L + RS_TILE - 1) / RS_TILE);
-    const unsigned grid = std::min<uint32_t>(ntiles, 152u * 8u);
+    uint32_t per;
+    const uint32_t runs = sort_runs(L, &per);
     const char *hname = aux ? "rs_hist_kernel.aux" : "rs_hist_kernel";
     const char *sname = aux ? "rs_scatter_kernel.aux" : "rs_scatter_kernel";
     uint64_t *src = keys, *dst = ws.tmp.p;
     for (uint32_t shift = lo; shift < hi; shift += 8) {
-        PADO_LAUNCH(hname, s, rs_hist_kernel<<<grid, RS_THREADS, 0, s>>>(src, L, shift, ntiles, ws.counts.p));
-        exclusive_scan(ws.counts.p, (uint64_t)256 * ntiles, ws.sums.p, s);
-        PADO_LAUNCH(sname, s, rs_scatter_kernel<<<grid, RS_THREADS, 0, s>>>(src, dst, L, shift, ntiles, ws.counts.p));
+        PADO_LAUNCH(hname, s, rs_hist_kernel<<<runs, RS_THREADS, 0, s>>>(src, L, shift, per, ws.counts.p));
+        PADO_LAUNCH("rs_scan_kernel", s, rs_scan_kernel<<<256, RS_THREADS, 0, s>>>(ws.counts.p, runs, ws.totals.p));
+        if (eo && shift + 8 >= hi)
+            PADO_LAUNCH(sname, s,
+                        rs_scatter_kernel<true><<<runs, RS_THREADS, 0, s>>>(src, dst, L, shift, per, ws.counts.p,
+                                                                            ws.totals.p, *eo));
+        else
+            PADO_LAUNCH(sname, s,
+                        rs_scatter_kernel<false><<<runs, RS_THREADS, 0, s>>>(src, dst, L, shift, per, ws.counts.p,
+                                                                             ws.totals.p, EntryOut{}));
         std::swap(src, dst);
     }
     return src;
@@ -397,28 +488,40 @@ __global__ void __launch_bounds__(256) unique_scatter_kernel(const uint64_t *key
 // claimed by the first vertex that hashes there; vertices that find their
 // slot taken add to global memory directly.  The heavy vertices of a skewed
 // graph claim their slots early (they are most of the endpoints) and then
-// cost one global atomic per block instead of one per endpoint.
-constexpr uint32_t DEG_SLOTS = 2048;
+// cost one global atomic per block instead of one per endpoint.  Bound by the
+// global atomics of the rest, so the table takes most of an SM's shared memory
+// (one block of 1,024 threads per SM): 33.5M endpoints of R-MAT s20 samples
+// take 190 us with 16,384 slots, 249 us with 8,192 (two blocks), 418 us with
+// 2,048 (eight blocks of 256).
+constexpr uint32_t DEG_LOG = 14, DEG_SLOTS = 1u << DEG_LOG;
+constexpr int DEG_THREADS = 1024;
+constexpr uint32_t DEG_SMEM = DEG_SLOTS * 8;
 
 __device__ __forceinline__ void count_endpoint(uint32_t a, uint32_t *cid, uint32_t *ccnt, uint32_t *deg)
 {
-    const uint32_t slot = (a * 2654435761u) >> 21;  // top 11 bits: DEG_SLOTS slots
-    const uint32_t old = atomicCAS(&cid[slot], 0xffffffffu, a);
-    if (old == 0xffffffffu || old == a)
+    const uint32_t slot = (a * 2654435761u) >> (32 - DEG_LOG);
+    uint32_t old = *(volatile uint32_t *)&cid[slot];
+    if (old == 0xffffffffu) {
+        old = atomicCAS(&cid[slot], 0xffffffffu, a);
+        if (old == 0xffffffffu) old = a;
+    }
+    if (old == a)
         atomicAdd(&ccnt[slot], 1u);
     else
         atomicAdd(&deg[a], 1u);
 }
 
-__global__ void __launch_bounds__(256) degree_kernel(const uint32_t *u, const uint32_t *v, uint64_t m, uint32_t n,
-                                                     uint32_t *deg, uint32_t *bad)
+__global__ void __launch_bounds__(DEG_THREADS) degree_kernel(const uint32_t *u, const uint32_t *v, uint64_t m,
+                                                             uint32_t n, uint32_t *deg, uint32_t *bad)
 {
-    __shared__ uint32_t cid[DEG_SLOTS], ccnt[DEG_SLOTS];
+    extern __shared__ uint32_t deg_tab[];
+    uint32_t *cid = deg_tab, *ccnt = deg_tab + DEG_SLOTS;
     for (uint32_t k = threadIdx.x; k < DEG_SLOTS; k += blockDim.x) {
         cid[k] = 0xffffffffu;
         ccnt[k] = 0;
     }
     __syncthreads();
+#pragma unroll 4
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t a = u[e], b = v[e];
         if (a >= n || b >= n) {
@@ -431,6 +534,18 @@ __global__ void __launch_bounds__(256) degree_kernel(const uint32_t *u, const ui
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < DEG_SLOTS; k += blockDim.x)
         if (ccnt[k]) atomicAdd(&deg[cid[k]], ccnt[k]);
+}
+
+// A block handles at least four edges per thread, so that small inputs do not
+// pay for tables they hardly use.
+void count_degrees(const uint32_t *u, const uint32_t *v, uint64_t m, uint32_t n, uint32_t *deg, uint32_t *bad,
+                   cudaStream_t s)
+{
+    if (!m) return;
+    PADO_CUDA(cudaFuncSetAttribute(degree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEG_SMEM));
+    PADO_LAUNCH("degree_kernel", s,
+                degree_kernel<<<grid_for((m + 3) / 4, DEG_THREADS, 152u), DEG_THREADS, DEG_SMEM, s>>>(u, v, m, n, deg,
+                                                                                                      bad));
 }
 
 __global__ void __launch_bounds__(256) max_deg_kernel(const uint32_t *deg, uint32_t n, uint32_t *mx)
@@ -476,17 +591,6 @@ __global__ void __launch_bounds__(256) entry_key_kernel(const uint32_t *u, const
         const uint64_t lw = 255u - (w ? w[e] : 0u);
         keys[2 * e] = ra << (bits + 8) | (dmask - rb) << 8 | lw;
         keys[2 * e + 1] = rb << (bits + 8) | (dmask - ra) << 8 | lw;
-    }
-}
-
-__global__ void __launch_bounds__(256) extract_kernel(const uint64_t *keys, uint64_t L, uint32_t bits, uint32_t *adj,
-                                                      uint8_t *w)
-{
-    const uint64_t dmask = (1ull << bits) - 1;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < L; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k = keys[i];
-        adj[i] = (uint32_t)(dmask - ((k >> 8) & dmask));
-        if (w) w[i] = (uint8_t)(255u - (uint32_t)(k & 255u));
     }
 }
 
@@ -930,9 +1034,7 @@ IngestResult ingest_edges(uint64_t m, const uint32_t *du, const uint32_t *dv, co
         PBuf<uint32_t> deg(std::max<uint32_t>(n, 1), s);
         deg.zero();
         scal.zero();
-        if (m)
-            PADO_LAUNCH("degree_kernel", s,
-                        degree_kernel<<<grid_for(m, 256, 152u * 8u), 256, 0, s>>>(du, dv, m, n, deg.p, scal.p));
+        count_degrees(du, dv, m, n, deg.p, scal.p, s);
         PADO_CHECK(read_back(scal.p, s) == 0, PADO_E_ARG, "edge endpoint out of range");
         scal.zero();
         if (n) PADO_LAUNCH("max_deg_kernel", s, max_deg_kernel<<<grid_for(n, 256), 256, 0, s>>>(deg.p, n, scal.p));
@@ -965,9 +1067,8 @@ IngestResult ingest_edges(uint64_t m, const uint32_t *du, const uint32_t *dv, co
         PADO_LAUNCH("entry_key_kernel", s,
                     entry_key_kernel<<<grid_for(m, 256), 256, 0, s>>>(du, dv, dw, m, r.rank.p, bits, keys.p));
         // after dedupe no (src, dst) pair repeats, so the weight byte needs no pass
-        const uint64_t *sorted = radix_sort(keys.p, L, dw && !dedupe ? 0u : 8u, 2 * bits + 8, ws, s);
-        PADO_LAUNCH("extract_kernel", s,
-                    extract_kernel<<<grid_for(L, 256), 256, 0, s>>>(sorted, L, bits, adj_out, dw ? w_out : nullptr));
+        const EntryOut eo{bits, adj_out, dw ? w_out : nullptr};
+        radix_sort(keys.p, L, dw && !dedupe ? 0u : 8u, 2 * bits + 8, ws, s, false, &eo);
     }
     PADO_CUDA(cudaStreamSynchronize(s));
     return r;
@@ -1034,9 +1135,8 @@ DevGraph prepare_csr(uint32_t n, const uint64_t *off, const uint32_t *adj, const
                         g.off.p));
         PBuf<uint32_t> osums(scan_sums_needed((uint64_t)n + 1), s);
         exclusive_scan(g.off.p, (uint64_t)n + 1, osums.p, s);
-        const uint64_t *sorted = radix_sort(keys.p, m, w ? 0u : 8u, 2 * bits + 8, ws, s);
-        PADO_LAUNCH("extract_kernel", s,
-                    extract_kernel<<<grid_for(m, 256), 256, 0, s>>>(sorted, m, bits, g.adj.p, w ? g.w.p : nullptr));
+        const EntryOut eo{bits, g.adj.p, w ? g.w.p : nullptr};
+        radix_sort(keys.p, m, w ? 0u : 8u, 2 * bits + 8, ws, s, false, &eo);
     } else {
         g.off.fill_bytes(0, s);
     }
@@ -1157,9 +1257,7 @@ void entry_degrees(uint64_t m, const uint32_t *du, const uint32_t *dv, uint32_t 
 {
     PADO_CUDA(cudaMemsetAsync(deg, 0, (size_t)n * 4, s));
     PADO_CUDA(cudaMemsetAsync(scal, 0, 4, s));
-    if (m)
-        PADO_LAUNCH("degree_kernel", s,
-                    degree_kernel<<<grid_for(m, 256, 152u * 8u), 256, 0, s>>>(du, dv, m, n, deg, scal));
+    count_degrees(du, dv, m, n, deg, scal, s);
     PADO_CHECK(read_back(scal, s) == 0, PADO_E_ARG, "edge endpoint out of range");
 }
 
