@@ -30,12 +30,12 @@
 // by the same stable LSD radix sort and the adjacency and weights are read
 // back out of them.
 //
-// The radix sort: 8-bit digits, tiles of 4096 keys, three kernels per digit
-// -- per-tile digit counts, one exclusive scan over the (digit, tile) matrix,
-// and a scatter in which each block ranks its tile's keys by digit (lanes
-// holding the same digit ranked with __match_any_sync, warps by a prefix over
-// the block), reorders the tile in shared memory and writes every digit's
-// run to its global position in coalesced stores.
+// The radix sort: 8-bit digits, tiles of 3584 keys, a run of tiles per block,
+// three kernels per digit -- digit counts per run, an exclusive scan of every
+// digit's counts, and a scatter in which a block ranks a tile's keys by digit
+// (lanes holding the same digit found by ballots, warps by a prefix over the
+// block), reorders the tile in shared memory and writes every digit's keys to
+// their global position in coalesced stores.
 
 #include <algorithm>
 #include <cstdio>
@@ -52,8 +52,8 @@ namespace {
 
 constexpr unsigned FULLW = 0xffffffffu;
 constexpr int RS_THREADS = 256;                  // radix sort block
-constexpr int RS_PER = 16;                       // keys per thread
-constexpr uint32_t RS_TILE = RS_THREADS * RS_PER;  // 4096 keys per tile
+constexpr int RS_PER = 14;                       // keys per thread
+constexpr uint32_t RS_TILE = RS_THREADS * RS_PER;  // 3584 keys per tile
 constexpr uint32_t TEXT_CHUNK = 16;              // bytes per thread when locating newlines
 
 // ---- scan -------------------------------------------------------------------
@@ -259,14 +259,15 @@ __global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const uint64_t *key
 
 // One block per digit: its counts become their exclusive prefix over the runs,
 // totals[d] their sum.
-__global__ void __launch_bounds__(RS_THREADS) rs_scan_kernel(uint32_t *counts, uint32_t nruns, uint32_t *totals)
+constexpr int RS_SCAN_THREADS = 1024;
+__global__ void __launch_bounds__(RS_SCAN_THREADS) rs_scan_kernel(uint32_t *counts, uint32_t nruns, uint32_t *totals)
 {
     uint32_t *c = counts + (uint64_t)blockIdx.x * nruns;
     uint32_t carry = 0;
-    for (uint32_t c0 = 0; c0 < nruns; c0 += RS_THREADS) {
+    for (uint32_t c0 = 0; c0 < nruns; c0 += RS_SCAN_THREADS) {
         const uint32_t i = c0 + threadIdx.x;
         uint32_t total;
-        const uint32_t pre = block_prefix<RS_THREADS>(i < nruns ? c[i] : 0u, &total);
+        const uint32_t pre = block_prefix<RS_SCAN_THREADS>(i < nruns ? c[i] : 0u, &total);
         if (i < nruns) c[i] = carry + pre;
         carry += total;
     }
@@ -281,13 +282,32 @@ struct EntryOut {
     uint8_t *w = nullptr;
 };
 
-// Stable scatter of one digit.  Warp w owns keys [512 w, 512 w + 512) of a
+// Lanes of the warp whose 8-bit digit is `dig`.
+__device__ __forceinline__ uint32_t digit_peers(uint32_t dig)
+{
+    uint32_t m = FULLW;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const uint32_t v = __ballot_sync(FULLW, dig >> b & 1u);
+        m &= dig >> b & 1u ? v : ~v;
+    }
+    return m;
+}
+
+// Stable scatter of one digit.  Warp w owns keys [448 w, 448 w + 448) of a
 // tile, 32 per round; a key's place among the tile's keys with its digit is
 // (keys of lower warps) + (keys of earlier rounds of its warp) + (lower lanes
-// of its round), which is its input order.  A thread's 16 keys are loaded
-// before any ranking so that their loads are in flight together.  A block
-// takes its run tile by tile and moves each digit's position on as it goes, so
-// the pass needs counts per run only, not per tile.
+// of its round), which is its input order.  A thread's keys are loaded before
+// any ranking so that their loads are in flight together.  A block takes its
+// run tile by tile and moves each digit's position on as it goes, so the pass
+// needs counts per run only, not per tile.
+//
+// What bounds it: the shared-memory pipe (82-89% busy with __match_any_sync
+// for the peers, ranks kept in shared memory and a table of digit starts), so
+// peers come from eight ballots, ranks stay in registers (14 keys per thread:
+// 16 spill at 4 blocks per SM) and a warp's first slots already hold the digit
+// starts.  33.5M keys per pass: 211 us before, 172 us now (3.1 TB/s of keys
+// read and written, 46% of the copy bandwidth).
 template <bool ENTRIES>
 __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_t *in, uint64_t *out, uint64_t L,
                                                                 uint32_t shift, uint32_t per,
@@ -296,9 +316,7 @@ __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_
 {
     constexpr int NW = RS_THREADS / 32;
     __shared__ uint64_t sk[RS_TILE];      // the tile, reordered by digit
-    __shared__ uint16_t slr[RS_TILE];     // rank of key i among its warp's keys with its digit
-    __shared__ uint16_t wcnt[NW][256];    // per warp and digit: count, then prefix over warps
-    __shared__ uint32_t dstart[256];      // first slot of each digit in the reordered tile
+    __shared__ uint16_t wcnt[NW][256];    // per warp and digit: count, then first slot in the reordered tile
     __shared__ uint32_t gbase[256];       // global position of slot 0 as each digit's run sees it
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
@@ -311,6 +329,7 @@ __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_
         const uint32_t cnt = (uint32_t)min(run1 - t0, (uint64_t)RS_TILE);
         const uint32_t i0 = wl * (RS_PER * 32) + lane;
         uint64_t key[RS_PER];
+        uint32_t rank[RS_PER / 2];  // 16 bits each: place among the warp's keys with the digit
 #pragma unroll
         for (int r = 0; r < RS_PER; ++r) key[r] = i0 + r * 32 < cnt ? in[t0 + i0 + r * 32] : 0ull;
 #pragma unroll
@@ -318,37 +337,38 @@ __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < RS_PER; ++r) {
-            const uint32_t i = i0 + r * 32;
-            const bool live = i < cnt;
-            const uint32_t dig = live ? (uint32_t)((key[r] >> shift) & 255u) : 256u + lane;  // idle lanes alone
-            const uint32_t peers = __match_any_sync(FULLW, dig);
-            if (live) slr[i] = (uint16_t)(wcnt[wl][dig] + __popc(peers & below));
+            const uint32_t dig = (uint32_t)(key[r] >> shift) & 255u;
+            const uint32_t peers = digit_peers(dig) & __ballot_sync(FULLW, i0 + r * 32 < cnt);
+            const uint32_t before = wcnt[wl][dig];
             __syncwarp();
-            if (live && (peers & below) == 0) wcnt[wl][dig] += (uint16_t)__popc(peers);
+            const uint32_t place = before + __popc(peers & below);
+            if (r & 1)
+                rank[r / 2] |= place << 16;
+            else
+                rank[r / 2] = place;
+            // the first live lane of a digit counts its round
+            if ((peers & below) == 0 && i0 + r * 32 < cnt) wcnt[wl][dig] = (uint16_t)(before + __popc(peers));
             __syncwarp();
         }
         __syncthreads();
-        // thread d: prefix of digit d over the warps, and the digit's total
+        // thread d: counts of digit d over the warps -> first slots
         uint32_t tot = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) tot += wcnt[w][threadIdx.x];
+        uint32_t slot = block_prefix<RS_THREADS>(tot, &unused);
+        gbase[threadIdx.x] = pos - slot;
+        pos += tot;
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
             const uint32_t c = wcnt[w][threadIdx.x];
-            wcnt[w][threadIdx.x] = (uint16_t)tot;
-            tot += c;
+            wcnt[w][threadIdx.x] = (uint16_t)slot;
+            slot += c;
         }
-        const uint32_t ds = block_prefix<RS_THREADS>(tot, &unused);
-        dstart[threadIdx.x] = ds;
-        gbase[threadIdx.x] = pos - ds;
-        pos += tot;
         __syncthreads();
 #pragma unroll
-        for (int r = 0; r < RS_PER; ++r) {
-            const uint32_t i = i0 + r * 32;
-            if (i < cnt) {
-                const uint32_t dig = (uint32_t)((key[r] >> shift) & 255u);
-                sk[dstart[dig] + wcnt[wl][dig] + slr[i]] = key[r];
-            }
-        }
+        for (int r = 0; r < RS_PER; ++r)
+            if (i0 + r * 32 < cnt)
+                sk[wcnt[wl][(uint32_t)(key[r] >> shift) & 255u] + (rank[r / 2] >> (16 * (r & 1)) & 0xffffu)] = key[r];
         __syncthreads();
         const uint64_t dmask = (1ull << eo.bits) - 1;
         for (uint32_t p = threadIdx.x; p < cnt; p += RS_THREADS) {
@@ -365,9 +385,11 @@ __global__ void __launch_bounds__(RS_THREADS, 4) rs_scatter_kernel(const uint64_
     }
 }
 
-// Runs of a sort of L keys: one per resident block of the scatter, or one per
-// tile where there are fewer.
-constexpr uint32_t RS_MAX_RUNS = 152u * 4u;
+// Runs of a sort of L keys: up to four waves of resident scatter blocks, so
+// that the last wave's idle SMs cost little (one wave: 979 us for the five
+// passes of the 33.5M-key sort, two 913, four 861), or one per tile where
+// there are fewer.
+constexpr uint32_t RS_MAX_RUNS = 152u * 4u * 4u;
 
 uint32_t sort_runs(uint64_t L, uint32_t *per)
 {
@@ -404,7 +426,7 @@ uint64_t *radix_sort(uint64_t *keys, uint64_t L, uint32_t lo, uint32_t hi, SortS
     uint64_t *src = keys, *dst = ws.tmp.p;
     for (uint32_t shift = lo; shift < hi; shift += 8) {
         PADO_LAUNCH(hname, s, rs_hist_kernel<<<runs, RS_THREADS, 0, s>>>(src, L, shift, per, ws.counts.p));
-        PADO_LAUNCH("rs_scan_kernel", s, rs_scan_kernel<<<256, RS_THREADS, 0, s>>>(ws.counts.p, runs, ws.totals.p));
+        PADO_LAUNCH("rs_scan_kernel", s, rs_scan_kernel<<<256, RS_SCAN_THREADS, 0, s>>>(ws.counts.p, runs, ws.totals.p));
         if (eo && shift + 8 >= hi)
             PADO_LAUNCH(sname, s,
                         rs_scatter_kernel<true><<<runs, RS_THREADS, 0, s>>>(src, dst, L, shift, per, ws.counts.p,

@@ -249,3 +249,25 @@ def test_scratch_cache_keeps_results(pado):
             same(got, grank, want, wrank, "cached scratch")
     finally:
         _lib.check(_lib.lib.pado_set_scratch_cache(0))
+
+
+@pytest.mark.parametrize("edges", [1, 16, 447, 448, 449, 1791, 1792, 1793, 3584 * 152 * 8 - 1, 3584 * 152 * 8 + 1])
+def test_entry_sort_tile_edges(cuda_ok, edges):
+    """Entry counts (two per edge) around a warp's share, a tile and the point
+    where a block's run takes more than one tile; few vertices make digits
+    heavily repeated, many make them spread."""
+    from parallel_distance_oracle_gb300 import pado
+    rng = np.random.Generator(np.random.PCG64(edges))
+    for n in (3, 70_001):
+        u = (n * rng.random(edges) ** 3).astype(np.uint32)
+        v = rng.integers(0, n, edges).astype(np.uint32)
+        w = rng.integers(0, 256, edges).astype(np.uint8)
+        g, rank = pado.graph_ingest(u, v, w, n=n)
+        src, dst = np.concatenate([u, v]), np.concatenate([v, u])
+        deg = np.bincount(src, minlength=n)
+        want = np.empty(n, np.int64)
+        want[np.lexsort((np.arange(n), -deg))] = np.arange(n)
+        assert np.array_equal(rank, want)
+        order = np.lexsort((-np.concatenate([w, w]).astype(np.int64), -want[dst], want[src]))
+        assert np.array_equal(g.adj, want[dst][order]) and np.array_equal(g.w, np.concatenate([w, w])[order])
+        assert np.array_equal(np.diff(g.off.astype(np.int64)), deg[np.argsort(want)])
