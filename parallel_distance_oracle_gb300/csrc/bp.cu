@@ -376,30 +376,30 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
     cudaEvent_t e0, e1;
     PADO_CUDA(cudaEventCreate(&e0));
     PADO_CUDA(cudaEventCreate(&e1));
-    uint32_t *h_cnt = nullptr;
+    uint32_t h_cnt[4] = {};
     try {
-        PADO_CUDA(cudaMallocHost((void **)&h_cnt, 8 * sizeof(uint32_t)));
         PADO_CUDA(cudaEventRecord(e0, s));
         // rows start unreached: level 255, empty sets (also the rows of slots no graph has a root for)
         PADO_CUDA(cudaMemsetAsync(d_bpd, 0xff, (uint64_t)n * K, s));
         PADO_CUDA(cudaMemsetAsync(d_bps, 0, (uint64_t)n * K * 16, s));
-        DBuf<unsigned long long> reach(n);
-        DBuf<LevelMask> lm0(n), lm1(n);
-        DBuf<uint32_t> cstamp(n), fstamp(n), cnts(8), status(1);
+        Arena zeros, ws;
+        DBuf<unsigned long long> reach;
+        DBuf<LevelMask> lm0, lm1;
+        DBuf<uint32_t> cstamp, fstamp, cnts, status;
         DBuf<uint32_t> fl[2], fh[2], cl, ch;
-        for (int i = 0; i < 2; ++i) {
-            fl[i].alloc(n);
-            fh[i].alloc(n);
-        }
-        cl.alloc(n);
-        ch.alloc(n);
-        reach.fill_bytes(0, s);
+        zeros.add(reach, n);
+        zeros.add(cstamp, n);
+        zeros.add(cnts, 8);
+        zeros.add(status, 1);
+        ws.add(lm0, n);
+        ws.add(lm1, n);
+        for (DBuf<uint32_t> *x : {&fstamp, &fl[0], &fl[1], &fh[0], &fh[1], &cl, &ch}) ws.add(*x, n);
+        zeros.commit();
+        ws.commit();
+        zeros.mem.fill_bytes(0, s);
         // empty masks stamped with a level no BFS reaches
         PADO_LAUNCH("bp_init_kernel", s, bp_init_kernel<<<grid_for(n, 256), 256, 0, s>>>(lm0.p, lm1.p, n));
-        cstamp.fill_bytes(0, s);
         fstamp.fill_bytes(0xff, s);
-        status.fill_bytes(0, s);
-        cnts.fill_bytes(0, s);
         MsState st{n, K, g.off.p, g.adj.p, d_bpd, reinterpret_cast<ulonglong2 *>(d_bps), reach.p,
                    {lm0.p, lm1.p}, cstamp.p, fstamp.p, work_counters()};
 
@@ -430,11 +430,16 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
             PADO_CUDA(cudaEventElapsedTime(&res.ms, e0, e1));
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
-            cudaFreeHost(h_cnt);
             return res;
         }
-        DBuf<uint32_t> d_ss(ss.size()), d_sv(sv.size()), d_sl(sl.size());
-        DBuf<uint64_t> d_sb(sb.size());
+        Arena seed_ws;
+        DBuf<uint32_t> d_ss, d_sv, d_sl;
+        DBuf<uint64_t> d_sb;
+        seed_ws.add(d_ss, ss.size());
+        seed_ws.add(d_sv, sv.size());
+        seed_ws.add(d_sl, sl.size());
+        seed_ws.add(d_sb, sb.size());
+        seed_ws.commit();
         d_ss.upload(ss.data(), ss.size(), s);
         d_sv.upload(sv.data(), sv.size(), s);
         d_sl.upload(sl.data(), sl.size(), s);
@@ -481,12 +486,10 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        if (h_cnt) cudaFreeHost(h_cnt);
         throw;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaFreeHost(h_cnt);
     return res;
 }
 

@@ -184,6 +184,8 @@ T read_back(const T *d, cudaStream_t s)
     return x;
 }
 
+}  // namespace
+
 // Scratch comes from a memory pool of this library's own (one per device),
 // allocated and freed in stream order: a call's buffers are reused by its
 // later steps without device-wide synchronisation, and up to
@@ -209,6 +211,8 @@ cudaMemPool_t scratch_pool()
     pools[dev] = pool;
     return pool;
 }
+
+namespace {
 
 template <typename T>
 struct PBuf {

@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <functional>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -83,19 +84,20 @@ __device__ __forceinline__ T &dbg_ref(T *p, uint64_t i, uint64_t lim, uint32_t s
 void alloc_point();
 void alloc_live(int delta);
 
-// Owning device buffer.
+// Owning device buffer (or a part of an Arena, which then owns it).
 template <typename T>
 struct DBuf {
     T *p = nullptr;
     size_t n = 0;
+    bool own = true;
     DBuf() = default;
     explicit DBuf(size_t count) { alloc(count); }
     DBuf(const DBuf &) = delete;
     DBuf &operator=(const DBuf &) = delete;
-    DBuf(DBuf &&o) noexcept : p(o.p), n(o.n) { o.p = nullptr; o.n = 0; }
+    DBuf(DBuf &&o) noexcept : p(o.p), n(o.n), own(o.own) { o.p = nullptr; o.n = 0; }
     DBuf &operator=(DBuf &&o) noexcept
     {
-        if (this != &o) { release(); p = o.p; n = o.n; o.p = nullptr; o.n = 0; }
+        if (this != &o) { release(); p = o.p; n = o.n; own = o.own; o.p = nullptr; o.n = 0; }
         return *this;
     }
     ~DBuf() { release(); }
@@ -124,12 +126,13 @@ struct DBuf {
     }
     void release()
     {
-        if (p) {
+        if (p && own) {
             cudaFree(p);
             alloc_live(-1);
         }
         p = nullptr;
         n = 0;
+        own = true;
     }
     size_t bytes() const { return n * sizeof(T); }
     void upload(const T *h, size_t count, cudaStream_t s = 0)
@@ -145,6 +148,35 @@ struct DBuf {
         if (n) PADO_CUDA(cudaMemsetAsync(p, v, bytes(), s));
     }
 };
+
+// Many buffers in one device allocation: add() them, then commit().  A small
+// build's time is mostly host calls, and an allocation and release cost 9 us
+// each pair (75 us from a few MB on).  The arena outlives its buffers' use.
+struct Arena {
+    DBuf<uint8_t> mem;
+    size_t bytes = 0;
+    std::vector<std::function<void(uint8_t *)>> parts;
+    template <typename T>
+    void add(DBuf<T> &b, size_t count)
+    {
+        b.release();
+        b.own = false;
+        b.n = count;
+        parts.push_back([&b, at = bytes](uint8_t *base) { b.p = reinterpret_cast<T *>(base + at); });
+        bytes += (count * sizeof(T) + 255) / 256 * 256;
+    }
+    void commit()
+    {
+        mem.alloc(std::max<size_t>(bytes, 1));
+        for (auto &set : parts) set(mem.p);
+        parts.clear();
+    }
+};
+
+// The tables of a small build that may be replaced while it runs (the label
+// pool) share the arena up to this size; larger ones stay apart, so that growth
+// gives the old one back.
+constexpr uint64_t ARENA_POOL_BYTES = 64ull << 20;
 
 // Owning page-locked host buffer (DMA-able without a driver-side staging copy).
 template <typename T>

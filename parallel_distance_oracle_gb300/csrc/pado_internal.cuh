@@ -147,7 +147,9 @@ ReduceResult reduce_degree1(uint64_t m, const uint32_t *du, const uint32_t *dv, 
 ReduceResult reduce_equivalent(uint64_t m, const uint32_t *du, const uint32_t *dv, uint32_t n, cudaStream_t s,
                                uint8_t *redundant, uint32_t *new_id, uint64_t *kept);
 
-// Trims the ingest scratch pool of the current device to keep_bytes.
+// The current device's scratch pool (ingest.cu), for stream-ordered buffers.
+cudaMemPool_t scratch_pool();
+// Trims the scratch pool of the current device to keep_bytes.
 void release_scratch(uint64_t keep_bytes);
 // b[i] = a[i] for i < n (device arrays, stream-ordered).
 void widen_u32(const uint32_t *a, uint64_t n, uint64_t *b, cudaStream_t s);

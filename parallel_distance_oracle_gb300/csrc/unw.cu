@@ -307,32 +307,65 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     std::optional<HostPhase> release_phase;
     std::optional<HostPhase> alloc_phase(std::in_place, "label alloc");
 
-    DBuf<uint8_t> d_used(std::max<uint32_t>(n, 1));
+    const char *loop_env = std::getenv("PADO_LEVEL_LOOP");
+    const bool host_loop = loop_env && !strcmp(loop_env, "host");
+    const uint32_t nbatches = (uint32_t)(((uint64_t)n + B - 1) / B);
+    uint64_t cap = initial_pool_entries(n);
+    // one allocation that starts as zeros, one whose contents do not matter,
+    // and, unless they are small, the label pool and dist_matrix (255s; a
+    // second buffer for odd batches in the persistent loop) apart
+    Arena zeros, ws;
+    DBuf<uint32_t> pool_hub;
+    DBuf<uint8_t> pool_dist, dm;
+    const uint64_t dm_bytes = (host_loop ? 1 : 2) * (uint64_t)B * n;
+    if (cap * 5 + dm_bytes <= ARENA_POOL_BYTES) {
+        ws.add(pool_hub, cap);
+        ws.add(pool_dist, cap);
+        ws.add(dm, dm_bytes);
+    } else {
+        pool_hub.alloc(cap);
+        pool_dist.alloc(cap);
+        dm.alloc(dm_bytes);
+    }
+    DBuf<unsigned long long> pool_top;
+    DBuf<uint64_t> lab_off;
+    DBuf<LastGroup> last0, last1;  // stamp 0: no group yet
+    DBuf<uint32_t> lab_len, lab_cap, tail_stamp, ind_stamp, counters, status;
+    DBuf<LoopCtl> ctl;
+    zeros.add(pool_top, 1);
+    zeros.add(lab_off, n);
+    zeros.add(last0, n);
+    zeros.add(last1, n);
+    zeros.add(lab_len, n);
+    zeros.add(lab_cap, n);
+    zeros.add(tail_stamp, n);
+    zeros.add(ind_stamp, n);
+    zeros.add(counters, 8);
+    zeros.add(status, 1);
+    zeros.add(ctl, 1);
+    DBuf<uint8_t> d_used, bpmin;
+    DBuf<uint32_t> last_min0, last_min1, ind, front0, front1, tails, htails, tails2, htails3, retry, roots, rr, d_broots,
+        d_boff;
+    ws.add(d_used, std::max<uint32_t>(n, 1));
+    ws.add(bpmin, std::max<uint32_t>(n, 1));
+    ws.add(last_min0, n);
+    ws.add(last_min1, n);
+    ws.add(ind, (uint64_t)n * words);
+    for (DBuf<uint32_t> *x : {&front0, &front1, &tails, &htails, &retry}) ws.add(*x, n);
+    ws.add(roots, B);
+    if (!host_loop) {
+        ws.add(tails2, n);
+        ws.add(htails3, n);
+        ws.add(rr, B);
+        ws.add(d_broots, std::max<uint32_t>(n, 1));
+        ws.add(d_boff, (uint64_t)nbatches + 1);
+    }
+    zeros.commit();
+    ws.commit();
+    zeros.mem.fill_bytes(0, s);
+    dm.fill_bytes(0xff, s);
     d_used.upload(used.data(), n, s);
     if (n) PADO_LAUNCH("heavy_flag_kernel", s, heavy_flag_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, d_used.p));
-    uint64_t cap = initial_pool_entries(n);
-    DBuf<uint32_t> pool_hub(cap);
-    DBuf<uint8_t> pool_dist(cap);
-    DBuf<unsigned long long> pool_top(1);
-    DBuf<uint64_t> lab_off(n);
-    DBuf<LastGroup> last0(n), last1(n);
-    DBuf<uint32_t> lab_len(n), lab_cap(n), last_min0(n), last_min1(n);
-    DBuf<uint32_t> tail_stamp(n), ind_stamp(n);
-    DBuf<uint32_t> ind((uint64_t)n * words);
-    DBuf<uint8_t> dm((uint64_t)B * n);
-    DBuf<uint32_t> front0(n), front1(n), tails(n), htails(n), retry(n), counters(8), status(1);
-    DBuf<uint32_t> roots(B);
-    pool_top.fill_bytes(0, s);
-    lab_off.fill_bytes(0, s);
-    lab_len.fill_bytes(0, s);
-    lab_cap.fill_bytes(0, s);
-    last0.fill_bytes(0, s);  // stamp 0: no group yet
-    last1.fill_bytes(0, s);
-    tail_stamp.fill_bytes(0, s);
-    ind_stamp.fill_bytes(0, s);
-    dm.fill_bytes(0xff, s);
-    status.fill_bytes(0, s);
-    counters.fill_bytes(0, s);
 
     UnwDev d{};
     d.n = n;
@@ -350,7 +383,6 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     d.used = d_used.p;
     d.bpd = d_bpd;
     d.bps = d_bps;
-    DBuf<uint8_t> bpmin(std::max<uint32_t>(n, 1));
     if (K && n)
         PADO_LAUNCH("bpmin_kernel", s, bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p));
     d.bpmin = bpmin.p;
@@ -372,10 +404,9 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     d.status = status.p;
     d.work = work_counters();
 
-    // host-pinned mirror of the per-level counters
+    // the host-driven loop's mirror of the per-level counters
     struct Ctr { uint32_t front_next, tails, retry, status; unsigned long long top; };
-    Ctr *hc = nullptr;
-    PADO_CUDA(cudaMallocHost((void **)&hc, sizeof(Ctr)));
+    Ctr ctr{}, *hc = &ctr;
     uint32_t *c_front[2] = {counters.p + 0, counters.p + 1};
     uint32_t *c_tails = counters.p + 2, *c_retry = counters.p + 3, *c_htails = counters.p + 4;
     const uint32_t smem = pull_smem_bytes(words, B);
@@ -420,9 +451,6 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     const bool trace = std::getenv("PADO_TRACE") != nullptr;
     struct TraceRow { uint32_t b, levels; uint64_t tails, front; cudaEvent_t ev; };
     std::vector<TraceRow> trace_rows;
-    const uint32_t nbatches = (uint32_t)(((uint64_t)n + B - 1) / B);
-    const char *loop_env = std::getenv("PADO_LEVEL_LOOP");
-    const bool host_loop = loop_env && !strcmp(loop_env, "host");
     try {
         if (!host_loop && n) {
             // ---- persistent cooperative loop ----
@@ -435,22 +463,15 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
                     if (!used[r]) hb_roots.push_back(r);
                 hb_off[b + 1] = (uint32_t)hb_roots.size();
             }
-            DBuf<uint32_t> d_broots(std::max<size_t>(hb_roots.size(), 1)), d_boff(nbatches + 1);
             d_broots.upload(hb_roots.data(), hb_roots.size(), s);
             d_boff.upload(hb_off.data(), nbatches + 1, s);
-            DBuf<uint8_t> dm2((uint64_t)B * n);  // second dist_matrix buffer (odd batches)
-            dm2.fill_bytes(0xff, s);
-            DBuf<uint32_t> tails2(n), htails3(n);
-            DBuf<LoopCtl> ctl(1);
-            DBuf<uint32_t> rr(B);
             DBuf<unsigned long long> bns(trace ? nbatches : 1);
             const uint32_t level_cap = trace ? (1u << 22) : 0u;
             DBuf<unsigned long long> llog(trace ? 2ull * level_cap : 1);
-            ctl.fill_bytes(0, s);
             if (trace) bns.fill_bytes(0, s);
             // tail slots: the three light lists reuse the host loop's front and tail buffers
             LoopBufs bf{d_broots.p, d_boff.p, rr.p, {tails.p, front0.p, tails2.p}, {htails.p, front1.p, htails3.p},
-                        retry.p, {dm.p, dm2.p}, trace ? bns.p : nullptr, trace ? llog.p : nullptr, level_cap,
+                        retry.p, {dm.p, dm.p + (uint64_t)B * n}, trace ? bns.p : nullptr, trace ? llog.p : nullptr, level_cap,
                         nbatches};
             const void *kfn = (const void *)label_loop_kernel;
             PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -664,12 +685,10 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        cudaFreeHost(hc);
         throw;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaFreeHost(hc);
     release_phase.emplace("label release");
     return run;
 }

@@ -305,39 +305,51 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
         run.batches += x.nb;
     }
 
-    DBuf<uint8_t> d_used(std::max<uint32_t>(n, 1));
-    d_used.upload(used.data(), n, s);
-    if (n) PADO_LAUNCH("heavy_flag_kernel", s, heavy_flag_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, d_used.p));
     // Many small graphs carry more labels per vertex than one large sparse
     // one, and every growth stops the loop: start at 3x the one-graph pool.
     uint64_t cap = debug_pool_entries() ? initial_pool_entries(n)
                                         : std::min<uint64_t>(3 * initial_pool_entries(n), 1ull << 31);
     DBuf<uint32_t> pool_hub(cap);
     DBuf<uint8_t> pool_dist(cap);
-    DBuf<unsigned long long> pool_top(1);
-    DBuf<uint64_t> lab_off(n);
-    DBuf<LastGroup> last0(n), last1(n);
-    DBuf<uint32_t> lab_len(n), lab_cap(n), last_min0(n), last_min1(n);
-    DBuf<uint32_t> tail_stamp(n), ind_stamp(n);
-    DBuf<uint32_t> ind((uint64_t)n * words);
-    DBuf<uint8_t> dm(2ull * B * n);  // two buffers per graph, by batch
-    DBuf<uint32_t> tl0(n), tl1(n), tl2(n), th0(n), th1(n), th2(n), rretry(n), tretry(n), status(1);
-    DBuf<uint32_t> rq0b(n), rq1b(n), zq0b(n), zq1b(n), rr(n);
-    DBuf<GDesc> d_gd(G);
-    DBuf<uint16_t> d_gmap(std::max<uint32_t>(n, 1));
-    DBuf<uint32_t> d_broots(std::max<size_t>(broots.size(), 1)), d_bcnt(std::max<size_t>(bcnt.size(), 1));
-    DBuf<uint32_t> d_gbase(G + 1);
-    DBuf<ManyCtl> ctl(1);
-    pool_top.fill_bytes(0, s);
-    lab_off.fill_bytes(0, s);
-    lab_len.fill_bytes(0, s);
-    lab_cap.fill_bytes(0, s);
-    last0.fill_bytes(0, s);  // stamp 0: no group yet
-    last1.fill_bytes(0, s);
-    tail_stamp.fill_bytes(0, s);
-    ind_stamp.fill_bytes(0, s);
+    // everything else in three allocations: one that starts as zeros, one
+    // whose contents do not matter, and dist_matrix (two buffers per graph, by
+    // batch)
+    Arena zeros, ws;
+    DBuf<unsigned long long> pool_top;
+    DBuf<uint64_t> lab_off;
+    DBuf<LastGroup> last0, last1;  // stamp 0: no group yet
+    DBuf<uint32_t> lab_len, lab_cap, tail_stamp, ind_stamp, status;
+    zeros.add(pool_top, 1);
+    zeros.add(lab_off, n);
+    zeros.add(last0, n);
+    zeros.add(last1, n);
+    for (DBuf<uint32_t> *x : {&lab_len, &lab_cap, &tail_stamp, &ind_stamp}) zeros.add(*x, n);
+    zeros.add(status, 1);
+    DBuf<uint8_t> d_used, bpmin;
+    DBuf<uint32_t> last_min0, last_min1, ind, tl0, tl1, tl2, th0, th1, th2, rretry, tretry, rq0b, rq1b, zq0b, zq1b, rr;
+    DBuf<uint32_t> d_broots, d_bcnt, d_gbase;
+    DBuf<GDesc> d_gd;
+    DBuf<uint16_t> d_gmap;
+    DBuf<ManyCtl> ctl;
+    ws.add(d_used, std::max<uint32_t>(n, 1));
+    ws.add(bpmin, std::max<uint32_t>(n, 1));
+    ws.add(ind, (uint64_t)n * words);
+    for (DBuf<uint32_t> *x : {&last_min0, &last_min1, &tl0, &tl1, &tl2, &th0, &th1, &th2, &rretry, &tretry, &rq0b, &rq1b,
+                              &zq0b, &zq1b, &rr})
+        ws.add(*x, n);
+    ws.add(d_broots, std::max<size_t>(broots.size(), 1));
+    ws.add(d_bcnt, std::max<size_t>(bcnt.size(), 1));
+    ws.add(d_gbase, G + 1);
+    ws.add(d_gd, G);
+    ws.add(d_gmap, std::max<uint32_t>(n, 1));
+    ws.add(ctl, 1);
+    zeros.commit();
+    ws.commit();
+    zeros.mem.fill_bytes(0, s);
+    DBuf<uint8_t> dm(2ull * B * n);
     dm.fill_bytes(0xff, s);
-    status.fill_bytes(0, s);
+    d_used.upload(used.data(), n, s);
+    if (n) PADO_LAUNCH("heavy_flag_kernel", s, heavy_flag_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, d_used.p));
     d_gd.upload(hgd.data(), G, s);
     d_gmap.upload(hgmap.data(), n, s);
     d_broots.upload(broots.data(), broots.size(), s);
@@ -367,7 +379,6 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     d.used = d_used.p;
     d.bpd = d_bpd;
     d.bps = d_bps;
-    DBuf<uint8_t> bpmin(std::max<uint32_t>(n, 1));
     if (K && n)
         PADO_LAUNCH("bpmin_kernel", s, bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p));
     d.bpmin = bpmin.p;

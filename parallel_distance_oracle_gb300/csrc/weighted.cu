@@ -903,28 +903,39 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     uint64_t lcap = initial_log_entries(n, B);
     DBuf<uint32_t> pool_hub(cap);
     DBuf<int16_t> pool_dist(cap);
-    DBuf<unsigned long long> pool_top(1), log_top(2);
-    DBuf<uint64_t> lab_off(n), last_pos0(n), last_pos1(n);
-    DBuf<uint32_t> lab_len(n), lab_cap(n), last_cnt0(n), last_cnt1(n), last_min0(n), last_min1(n);
-    DBuf<uint32_t> act_stamp0(n), act_stamp1(n), tail_stamp(n), vq_len(n);
-    DBuf<int16_t> buf((uint64_t)B * n), vd((uint64_t)n * B), snap((uint64_t)B * B);
-    DBuf<uint64_t> rbase(B);
-    DBuf<uint32_t> rlen(B);
+    DBuf<int16_t> buf((uint64_t)B * n), vd((uint64_t)n * B);
     DBuf<uint16_t> vq((uint64_t)n * B);
-    DBuf<uint32_t> dt((uint64_t)n * B);
     DBuf<uint32_t> log0(lcap), log1(lcap);
-    DBuf<uint32_t> front0(n), front1(n), tails(n), retry(n), news(n), counters(8), status(1);
-    pool_top.fill_bytes(0, s);
-    log_top.fill_bytes(0, s);
-    lab_off.fill_bytes(0, s);
-    lab_len.fill_bytes(0, s);
-    lab_cap.fill_bytes(0, s);
-    act_stamp0.fill_bytes(0, s);
-    act_stamp1.fill_bytes(0, s);
-    tail_stamp.fill_bytes(0, s);
-    vq_len.fill_bytes(0, s);
-    dt.fill_bytes(0, s);       // stamp 0 never matches a batch (stamps start at 1)
-    status.fill_bytes(0, s);
+    // the per-vertex arrays in two allocations: one that starts as zeros
+    // (with dt: stamp 0 never matches a batch, stamps start at 1) and one
+    // whose contents do not matter
+    Arena zeros, ws;
+    DBuf<unsigned long long> pool_top, log_top;
+    DBuf<uint64_t> lab_off, last_pos0, last_pos1, rbase;
+    DBuf<uint32_t> lab_len, lab_cap, act_stamp0, act_stamp1, tail_stamp, vq_len, dt, status;
+    DBuf<uint32_t> last_cnt0, last_cnt1, last_min0, last_min1, rlen, front0, front1, tails, tails2, tails3, retry, news,
+        news2, rr, heavy, counters;
+    DBuf<int16_t> snap;
+    DBuf<WLoopCtl> ctl;
+    zeros.add(pool_top, 1);
+    zeros.add(log_top, 2);
+    zeros.add(lab_off, n);
+    for (DBuf<uint32_t> *x : {&lab_len, &lab_cap, &act_stamp0, &act_stamp1, &tail_stamp, &vq_len}) zeros.add(*x, n);
+    zeros.add(dt, (uint64_t)n * B);
+    zeros.add(status, 1);
+    zeros.add(ctl, 1);
+    ws.add(last_pos0, n);
+    ws.add(last_pos1, n);
+    for (DBuf<uint32_t> *x : {&last_cnt0, &last_cnt1, &last_min0, &last_min1, &front0, &front1, &tails, &tails2, &tails3,
+                              &retry, &news, &news2, &rr, &heavy})
+        ws.add(*x, n);
+    ws.add(rbase, B);
+    ws.add(rlen, B);
+    ws.add(counters, 8);
+    ws.add(snap, (uint64_t)B * B);
+    zeros.commit();
+    ws.commit();
+    zeros.mem.fill_bytes(0, s);
     for (DBuf<int16_t> *t : {&buf, &vd})
         if (t->n)
             PADO_LAUNCH("w_fill_inf_kernel", s,
@@ -971,8 +982,7 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     PADO_CUDA(cudaFuncSetAttribute(w_pull_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pull_smem));
 
     struct Ctr { uint32_t front_next, tails, retry, news; unsigned long long top; unsigned long long ltop[2]; };
-    Ctr *hc = nullptr;
-    PADO_CUDA(cudaMallocHost((void **)&hc, sizeof(Ctr)));
+    Ctr ctr{}, *hc = &ctr;
     uint32_t *c_front[2] = {counters.p + 0, counters.p + 1};
     uint32_t *c_tails = counters.p + 2, *c_retry = counters.p + 3, *c_news = counters.p + 4;
     uint32_t *fronts[2] = {front0.p, front1.p};
@@ -1025,9 +1035,6 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     try {
         PADO_CHECK(nbatches < 65535u, PADO_E_ARG, "more than 65534 batches");
         if (!host_loop && n) {
-            DBuf<WLoopCtl> ctl(1);
-            DBuf<uint32_t> tails2(n), tails3(n), news2(n), rr(n), heavy(n);
-            ctl.fill_bytes(0, s);
             WLoopBufs bf{{tails.p, tails2.p, tails3.p}, {news.p, news2.p}, rr.p, retry.p, heavy.p, nbatches};
             const void *kfn = (const void *)w_loop_kernel;
             PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pull_smem));
@@ -1171,12 +1178,10 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        cudaFreeHost(hc);
         throw;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaFreeHost(hc);
     return run;
 }
 
