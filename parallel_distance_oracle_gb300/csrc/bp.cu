@@ -22,10 +22,10 @@
 // one coalesced 16-byte load per lane and only for the slots where it matters;
 // the adjacency of a vertex is scanned once per level for all slots together
 // instead of once per slot.  Per level d:
-//   bp_sibling_kernel: each vertex v on level d (in any slot) ORs S^-1 of its
+//   sibling_phase: each vertex v on level d (in any slot) ORs S^-1 of its
 //       neighbours that share a level-d slot into S^0[v] (the sibling step),
 //       and lists the neighbours that still miss a slot v has on level d;
-//   bp_child_kernel: each listed vertex w takes, per slot it has not reached,
+//   child_phase: each listed vertex w takes, per slot it has not reached,
 //       the OR of S^-1 / S^0 over its neighbours on level d in that slot (the
 //       child step); slots so reached get level d+1 and put w on level d+1.
 // The child step pulls along the same edges the reference pushes along, and
@@ -37,6 +37,7 @@
 
 #include <algorithm>
 
+#include "grid_barrier.cuh"
 #include "pado_internal.cuh"
 
 namespace pado {
@@ -231,12 +232,12 @@ __device__ __forceinline__ void block_or(unsigned long long *sm, unsigned long l
 
 // Level d, sibling step over the frontier (heavy vertices by blocks, then
 // light ones by warps); also lists the child candidates of level d.
-__global__ void __launch_bounds__(BP_THREADS) bp_sibling_kernel(MsState st, VList front, uint32_t d, VList cand)
+__device__ void sibling_phase(const MsState &st, const VList &front, uint32_t d, const VList &cand,
+                              unsigned long long *sm, uint32_t *claim)
 {
-    __shared__ unsigned long long sm[BP_WARPS * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long bytes = 0;
-    const uint32_t hc = front.cnt[1];
+    const uint32_t hc = vload(&front.cnt[1]);
     for (uint32_t q = blockIdx.x; q < hc; q += gridDim.x) {
         const uint32_t v = front.heavy[q];
         const unsigned long long fv = level_bits(st, v, d);
@@ -250,9 +251,7 @@ __global__ void __launch_bounds__(BP_THREADS) bp_sibling_kernel(MsState st, VLis
             if (a1 && lane + 32 < (int)st.K) st.bps[row + lane + 32].y |= a1;
         }
     }
-    const uint32_t lc = front.cnt[0];
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < lc; q += nw) {
+    for_claimed<1>(vload(&front.cnt[0]), claim, [&](uint32_t q) {
         const uint32_t v = front.light[q];
         const unsigned long long fv = level_bits(st, v, d);
         unsigned long long a0 = 0, a1 = 0;
@@ -260,22 +259,17 @@ __global__ void __launch_bounds__(BP_THREADS) bp_sibling_kernel(MsState st, VLis
         const uint64_t row = (uint64_t)v * st.K;
         if (a0 && lane < (int)st.K) st.bps[row + lane].y |= a0;
         if (a1 && lane + 32 < (int)st.K) st.bps[row + lane + 32].y |= a1;
-    }
+    });
     if (st.work && lane == 0 && bytes) atomicAdd(&st.work[W_BP_SIB], bytes);
 }
 
 // Level d, child step over the candidates; builds the frontier of level d+1.
-__global__ void __launch_bounds__(BP_THREADS) bp_child_kernel(MsState st, VList cand, uint32_t d, VList next,
-                                                              uint32_t *status)
+__device__ void child_phase(const MsState &st, const VList &cand, uint32_t d, const VList &next,
+                            unsigned long long *sm, uint32_t *claim)
 {
-    __shared__ unsigned long long sm[BP_WARPS * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long bytes = 0;
-    if (d + 1 >= U8_INF) {
-        if ((cand.cnt[0] || cand.cnt[1]) && threadIdx.x == 0 && blockIdx.x == 0) atomicOr(status, ST_LEVEL_OVERFLOW);
-        return;
-    }
-    const uint32_t hc = cand.cnt[1];
+    const uint32_t hc = vload(&cand.cnt[1]);
     for (uint32_t q = blockIdx.x; q < hc; q += gridDim.x) {
         const uint32_t w = cand.heavy[q];
         const unsigned long long rw = st.reach[w];
@@ -289,17 +283,65 @@ __global__ void __launch_bounds__(BP_THREADS) bp_child_kernel(MsState st, VList 
         block_or(sm, a1.y, lane, warp);
         if (warp == 0) child_commit(st, w, rw, newm, a0, a1, d, next);  // newm is the same in every lane
     }
-    const uint32_t lc = cand.cnt[0];
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < lc; q += nw) {
+    for_claimed<1>(vload(&cand.cnt[0]), claim, [&](uint32_t q) {
         const uint32_t w = cand.light[q];
         const unsigned long long rw = st.reach[w];
         unsigned long long newm = 0;
         ulonglong2 a0 = make_ulonglong2(0, 0), a1 = make_ulonglong2(0, 0);
         child_range(st, w, rw, d, 0, 1, newm, a0, a1, bytes);
         child_commit(st, w, rw, newm, a0, a1, d, next);
-    }
+    });
     if (st.work && lane == 0 && bytes) atomicAdd(&st.work[W_BP_CHILD], bytes);
+}
+
+// All levels in one cooperative launch, a grid barrier after each step.  What
+// bounds small graphs is the turn-around of a level (two launches, two counter
+// copies, two clears and a wait took about 40 us; two barriers take 4), and a
+// union of many graphs has as many levels as its longest.  The frontier of
+// level d is in slot d % 3 (levels 0 and 1 are filled before the launch) and its
+// candidates are counted in cand[d & 1]; the leader clears each counter in
+// a step in which nobody reads or appends to it.
+struct BpCtl {
+    GridBar bar;
+    uint32_t front[3][2];  // light and heavy vertices of the frontier slots
+    uint32_t cand[2][2];
+    uint32_t sclaim[2], cclaim[2];  // claims of the sibling and child steps of level d, in slot d & 1
+    uint32_t levels, status;
+};
+
+struct BpLists {
+    uint32_t *light[3], *heavy[3];  // frontier slots
+    uint32_t *clight, *cheavy;
+};
+
+__global__ void __launch_bounds__(BP_THREADS, 4) bp_loop_kernel(MsState st, BpCtl *c, BpLists l)
+{
+    __shared__ unsigned long long sm[BP_WARPS * 32];
+    const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+    GridSync sync(&c->bar, &c->status);
+    for (uint32_t d = 0;; ++d) {
+        const uint32_t cur = d % 3, nxt = (d + 1) % 3, free_slot = (d + 2) % 3;
+        const VList front{l.light[cur], l.heavy[cur], c->front[cur]};
+        const VList next{l.light[nxt], l.heavy[nxt], c->front[nxt]};
+        const VList cand{l.clight, l.cheavy, c->cand[d & 1]};
+        if (leader) c->cclaim[(d + 1) & 1] = 0;  // level d - 1's child step is over
+        sibling_phase(st, front, d, cand, sm, &c->sclaim[d & 1]);
+        if (!sync.wait()) return;
+        if (leader) {
+            c->sclaim[d & 1] = 0;
+            // read by level d - 1 (frontier) and d - 1's child step (candidates)
+            c->front[free_slot][0] = c->front[free_slot][1] = 0;
+            c->cand[(d + 1) & 1][0] = c->cand[(d + 1) & 1][1] = 0;
+            c->levels = d + 1;
+        }
+        if (d + 1 >= U8_INF) {  // uniform: every block sees the same counters after the barrier
+            if (leader && (vload(&cand.cnt[0]) || vload(&cand.cnt[1]))) atomicOr(&c->status, ST_LEVEL_OVERFLOW);
+            return;
+        }
+        child_phase(st, cand, d, next, sm, &c->cclaim[d & 1]);
+        if (!sync.wait()) return;
+        if (vload(&next.cnt[0]) + vload(&next.cnt[1]) == 0) return;
+    }
 }
 
 __global__ void bp_init_kernel(LevelMask *a, LevelMask *b, uint32_t n)
@@ -376,7 +418,6 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
     cudaEvent_t e0, e1;
     PADO_CUDA(cudaEventCreate(&e0));
     PADO_CUDA(cudaEventCreate(&e1));
-    uint32_t h_cnt[4] = {};
     try {
         PADO_CUDA(cudaEventRecord(e0, s));
         // rows start unreached: level 255, empty sets (also the rows of slots no graph has a root for)
@@ -385,15 +426,15 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
         Arena zeros, ws;
         DBuf<unsigned long long> reach;
         DBuf<LevelMask> lm0, lm1;
-        DBuf<uint32_t> cstamp, fstamp, cnts, status;
-        DBuf<uint32_t> fl[2], fh[2], cl, ch;
+        DBuf<uint32_t> cstamp, fstamp;
+        DBuf<uint32_t> fl[3], fh[3], cl, ch;
+        DBuf<BpCtl> ctl;
         zeros.add(reach, n);
         zeros.add(cstamp, n);
-        zeros.add(cnts, 8);
-        zeros.add(status, 1);
         ws.add(lm0, n);
         ws.add(lm1, n);
-        for (DBuf<uint32_t> *x : {&fstamp, &fl[0], &fl[1], &fh[0], &fh[1], &cl, &ch}) ws.add(*x, n);
+        ws.add(ctl, 1);
+        for (DBuf<uint32_t> *x : {&fstamp, &fl[0], &fl[1], &fl[2], &fh[0], &fh[1], &fh[2], &cl, &ch}) ws.add(*x, n);
         zeros.commit();
         ws.commit();
         zeros.mem.fill_bytes(0, s);
@@ -451,38 +492,33 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
         fh[0].upload(f0[1].data(), f0[1].size(), s);
         fl[1].upload(f1[0].data(), f1[0].size(), s);
         fh[1].upload(f1[1].data(), f1[1].size(), s);
-        // cnts: [0,1] frontier d (light, heavy), [2,3] frontier d+1, [4,5] candidates
-        uint32_t init_cnt[8] = {(uint32_t)f0[0].size(), (uint32_t)f0[1].size(), (uint32_t)f1[0].size(),
-                                (uint32_t)f1[1].size(), 0, 0, 0, 0};
-        PADO_CUDA(cudaMemcpyAsync(cnts.p, init_cnt, sizeof(init_cnt), cudaMemcpyHostToDevice, s));
-        const unsigned grid = 152u * 8u;
-        int cur = 0;
-        uint32_t *ccur = cnts.p, *cnxt = cnts.p + 2, *ccand = cnts.p + 4;
-        uint32_t fsize = (uint32_t)(f0[0].size() + f0[1].size());
-        for (uint32_t d = 0; fsize > 0; ++d) {
-            const VList front{fl[cur].p, fh[cur].p, ccur};
-            const VList next{fl[cur ^ 1].p, fh[cur ^ 1].p, cnxt};
-            const VList cand{cl.p, ch.p, ccand};
-            PADO_LAUNCH("bp_sibling_kernel", s, bp_sibling_kernel<<<grid, BP_THREADS, 0, s>>>(st, front, d, cand));
-            PADO_LAUNCH("bp_child_kernel", s,
-                        bp_child_kernel<<<grid, BP_THREADS, 0, s>>>(st, cand, d, next, status.p));
-            ++res.levels;
-            PADO_CUDA(cudaMemcpyAsync(h_cnt, cnxt, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            PADO_CUDA(cudaMemcpyAsync(h_cnt + 2, status.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            PADO_CUDA(cudaMemsetAsync(ccur, 0, 2 * sizeof(uint32_t), s));
-            PADO_CUDA(cudaMemsetAsync(ccand, 0, 2 * sizeof(uint32_t), s));
-            PADO_CUDA(cudaStreamSynchronize(s));
-            if (h_cnt[2] & ST_LEVEL_OVERFLOW)
-                throw Error(PADO_E_OVERFLOW, "bit-parallel BFS reached level 255 (uint8 distance overflow)");
-            fsize = h_cnt[0] + h_cnt[1];
-            cur ^= 1;
-            std::swap(ccur, cnxt);
-        }
+        BpCtl h{};
+        h.front[0][0] = (uint32_t)f0[0].size();
+        h.front[0][1] = (uint32_t)f0[1].size();
+        h.front[1][0] = (uint32_t)f1[0].size();
+        h.front[1][1] = (uint32_t)f1[1].size();
+        ctl.upload(&h, 1, s);
+        int dev = 0, sms = 0, per_sm = 0;
+        PADO_CUDA(cudaGetDevice(&dev));
+        PADO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        PADO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_loop_kernel, BP_THREADS, 0));
+        PADO_CHECK(per_sm >= 1, PADO_E_CUDA, "bit-parallel loop kernel cannot be resident");
+        BpCtl *cp = ctl.p;
+        BpLists lists{{fl[0].p, fl[1].p, fl[2].p}, {fh[0].p, fh[1].p, fh[2].p}, cl.p, ch.p};
+        void *args[] = {&st, &cp, &lists};
+        PADO_LAUNCH("bp_loop_kernel", s,
+                    PADO_CUDA(cudaLaunchCooperativeKernel((const void *)bp_loop_kernel, sms * per_sm, BP_THREADS, args, 0,
+                                                          s)));
+        PADO_CUDA(cudaMemcpyAsync(&h, ctl.p, sizeof(h), cudaMemcpyDeviceToHost, s));
         PADO_LAUNCH("bp_finish_kernel", s,
                     bp_finish_kernel<<<grid_for((uint64_t)n * K, 256), 256, 0, s>>>(st));
         PADO_CUDA(cudaEventRecord(e1, s));
         PADO_CUDA(cudaEventSynchronize(e1));
         PADO_CUDA(cudaEventElapsedTime(&res.ms, e0, e1));
+        if (h.status & ST_BARRIER_TIMEOUT) throw Error(PADO_E_TIMEOUT, "bit-parallel loop: a grid barrier timed out");
+        if (h.status & ST_LEVEL_OVERFLOW)
+            throw Error(PADO_E_OVERFLOW, "bit-parallel BFS reached level 255 (uint8 distance overflow)");
+        res.levels = h.levels;
     } catch (...) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
