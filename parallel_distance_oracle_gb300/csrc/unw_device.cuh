@@ -1065,17 +1065,7 @@ __device__ void pull_phase(const UnwDev &d, const PullArgs &a, unsigned char *pu
     }
     WarpRegion wr = warp_region(pull_smem, d.words, d.B, threadIdx.x >> 5);
     if (a.tail_q) {
-        // the next claim is issued before the current tail is processed, so
-        // its latency is hidden; each warp over-claims once at the end
-        uint32_t q = 0;
-        if (lane == 0) q = atomicAdd(a.tail_q, 1u);
-        q = __shfl_sync(FULL, q, 0);
-        while (q < cnt) {
-            uint32_t nq = 0;
-            if (lane == 0) nq = atomicAdd(a.tail_q, 1u);
-            pull_light_tail(d, a, a.tails[q], wr, bytes);
-            q = __shfl_sync(FULL, nq, 0);
-        }
+        for_claimed<0>(cnt, a.tail_q, [&](uint32_t q) { pull_light_tail(d, a, a.tails[q], wr, bytes); });
     } else {
         const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
         for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < cnt; q += nw)

@@ -500,17 +500,7 @@ __device__ void w_pull_phase(const WDev &d, const uint32_t *tails, uint32_t cnt,
         if (nacc && next_tails) w_mark_head(d, t, mnacc, lid_cur + 1, next_tails, next_tails_cnt);
     };
     if (tq) {
-        // dynamic claiming: the next claim is issued before the current tail
-        // is processed; each warp over-claims once at the end
-        uint32_t q = 0;
-        if (lane == 0) q = atomicAdd(tq, 1u);
-        q = __shfl_sync(FULL, q, 0);
-        while (q < cnt) {
-            uint32_t nq = 0;
-            if (lane == 0) nq = atomicAdd(tq, 1u);
-            pull_tail(tails[q]);
-            q = __shfl_sync(FULL, nq, 0);
-        }
+        for_claimed<0>(cnt, tq, [&](uint32_t q) { pull_tail(tails[q]); });
     } else {
         for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < cnt; q += nw) pull_tail(tails[q]);
     }
