@@ -519,19 +519,23 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_pull_kernel(WDev d, con
 }
 
 // filter_out_labels (pado_weighted_unv_unp.h:1052-1184) on pre-filter values
-// for the temporary labels i0 .. i0 + 31 of v (one per lane): label c is
-// dropped, by setting bit 15 of its vq slot, when some root r < c of v's list
-// has d(v, r) <= d(v, c), d(c, r) <= d(v, c) and d(v, r) + d(c, r) <= d(v, c),
-// d(c, r) read from root c's temporary row.  v's list is taken 32 entries at
-// a time into the lanes and broadcast; each lane still looking keeps four
-// root-row gathers in flight.  Bit 15 is masked off wherever a slot is read,
-// so chunks of one v may run in different warps at once.
+// for the temporary labels i0 .. i0 + 31 of v: label c is dropped, by setting
+// bit 15 of its vq slot, when some root r < c of v's list has
+// d(v, r) <= d(v, c), d(c, r) <= d(v, c) and d(v, r) + d(c, r) <= d(v, c),
+// d(c, r) read from root c's temporary row.  v's list is walked 32 entries at
+// a time across the lanes; the labels still looking (bits of `pend`) are taken
+// four at a time, each gathering its own row at the 32 entries' roots, and
+// leave at the chunk that drops them (most leave in the first chunks: a lane per
+// label, all walking the whole list, took 9.1 ms for the first batch of
+// weighted R-MAT s18).  Bit 15 is masked off wherever a slot is read, so chunks
+// of one v may run in different warps at once.
 __device__ __forceinline__ void w_filter_chunk(const WDev &d, uint32_t v, uint32_t L, uint32_t i0, uint32_t s)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t B = d.B;
     uint16_t *vq = d.vq + (uint64_t)v * B;
     const int16_t *row = d.vd + (uint64_t)v * B;
+    const int16_t *rows = d.vd + (uint64_t)s * B;  // the roots' temporary rows
     const uint32_t i = i0 + lane;
     const bool valid = i < L;
     uint32_t c = 0;
@@ -540,33 +544,36 @@ __device__ __forceinline__ void w_filter_chunk(const WDev &d, uint32_t v, uint32
         c = vq[i] & 0x7fffu;
         dvc = row[c];
     }
-    const int16_t *crow = d.vd + (uint64_t)(s + c) * B;
-    bool filt = false;
-    for (uint32_t k0 = 0; k0 < L && __any_sync(FULL, valid && !filt); k0 += 32) {
-        const uint32_t kn = min(32u, L - k0);
-        const uint32_t rl = (uint32_t)lane < kn ? (uint32_t)(vq[k0 + lane] & 0x7fffu) : 0u;
-        const int32_t dl = (uint32_t)lane < kn ? (int32_t)row[rl] : 0;
-        for (uint32_t k = 0; k < kn; k += 4) {
-            uint32_t ru[4];
-            int32_t du[4], gu[4];
-            bool pu[4];
+    uint32_t pend = __ballot_sync(FULL, valid);
+    const uint32_t all = pend;
+    for (uint32_t k0 = 0; k0 < L && pend; k0 += 32) {
+        const bool in = k0 + lane < L;
+        const uint32_t rl = in ? (uint32_t)(vq[k0 + lane] & 0x7fffu) : 0u;
+        const int32_t dl = in ? (int32_t)row[rl] : 0;
+        uint32_t todo = pend;
+        while (todo) {
+            int jj[4];
+            int32_t mm[4], gg[4];
+            bool ok[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                ru[u] = __shfl_sync(FULL, rl, (int)(k + u) & 31);
-                du[u] = __shfl_sync(FULL, dl, (int)(k + u) & 31);
+                jj[u] = todo ? __ffs(todo) - 1 : -1;
+                todo &= todo - 1;  // (0 stays 0)
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                pu[u] = valid && !filt && k + u < kn && ru[u] < c && du[u] <= dvc;
-                gu[u] = pu[u] ? (int32_t)crow[ru[u]] : 0;
+                const uint32_t cu = __shfl_sync(FULL, c, jj[u] & 31);
+                mm[u] = __shfl_sync(FULL, dvc, jj[u] & 31);
+                ok[u] = jj[u] >= 0 && in && rl < cu && dl <= mm[u];
+                gg[u] = ok[u] ? (int32_t)rows[(uint64_t)cu * B + rl] : 0;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (pu[u] && gu[u] <= dvc && du[u] + gu[u] <= dvc) filt = true;
+                if (__ballot_sync(FULL, ok[u] && gg[u] <= mm[u] && dl + gg[u] <= mm[u])) pend &= ~(1u << jj[u]);
         }
     }
     __syncwarp();
-    if (valid && filt) vq[i] |= 0x8000u;
+    if ((all & ~pend) >> lane & 1u) vq[i] |= 0x8000u;
     __syncwarp();
 }
 
