@@ -47,7 +47,8 @@
 // and a host round trip each: start (the previous batch's roots' temporary
 // rows cleared; root tables; the roots mark the first round's tails), one
 // phase per round (the pull; a tail that accepts marks the next round's tails
-// itself; batch 0 takes a snapshot phase first), end (later batches: filter
+// itself; batch 0 takes a snapshot phase first; a round with heavy tails takes
+// a second phase for their checks and commits), end (later batches: filter
 // and commit each vertex in one phase; batch 0: filter, then the long lists'
 // remaining chunks over the grid, then commit).  It returns to the host only
 // to grow the round logs or the label pool (the failed tails or vertices are
@@ -57,6 +58,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <type_traits>
 
 #include "grid_barrier.cuh"
 #include "pado_internal.cuh"
@@ -67,6 +69,11 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int WPULL_WARPS = 4;
 constexpr int32_t RMIN_EMPTY = INT_MAX;
+// Tails of at least this degree are worked on by the whole grid: their heads
+// in items of WITEM adjacency entries, then a block each (see WTails).
+constexpr uint32_t WHEAVY_DEG = 512, WITEM = 64;
+constexpr uint32_t WHEAVY_BIT = 0x80000000u;  // of tail_stamp (rounds stay far below 2^31)
+constexpr int32_t HMIN_EMPTY = 0x7f7f7f7f;  // above every distance; a byte fill writes it
 
 struct WDev {
     uint32_t n, B;
@@ -92,13 +99,29 @@ struct WDev {
     uint32_t *last_cnt[2];
     uint32_t *last_min[2];
     uint32_t *act_stamp[2];  // by round parity: round id at which the vertex accepted roots
-    uint32_t *tail_stamp;
+    uint32_t *tail_stamp;  // round for which the vertex was last marked; top bit: heavy
     int16_t *snap;       // [B][B] rows of vertices < B at round start (batch 0)
     uint64_t *rbase;     // [B] pool position of root c's labels when its buf row was filled
     uint32_t *rlen;      // [B] their count (the row's reset reads these, not the live list,
                          // which a commit in the same phase may extend or move)
     uint32_t *status;
     unsigned long long *work;
+};
+
+// The tails of one round, in one of three slots by round mod 3: light ones, a
+// warp each, and, in the persistent loop, heavy ones with the items of their
+// adjacency.  A heavy tail's relaxations are min-reduced per item in shared
+// memory and then into its row of hmin; once all items are done a block
+// checks and commits it.  A warp alone would bound the round: in the first batch
+// of weighted R-MAT s18 a vertex of several thousand neighbours receives
+// hundreds of roots from each, and one round took 18.3 ms for 148,000 tails (5.8
+// now; the batch's eleven rounds 35.7 and 15.4).  Build loop by the limit: 57.5 ms
+// from degree 256 on, 55.7 from 512 or 1,024; items of 32 entries 55.9.
+struct WTails {
+    uint32_t *light, *light_cnt;
+    uint32_t *heavy = nullptr, *heavy_cnt = nullptr;
+    uint2 *items = nullptr;  // (index in `heavy`, item number)
+    uint32_t *items_cnt = nullptr;
 };
 
 __device__ __forceinline__ int32_t dt_get(const WDev &d, uint32_t t, uint32_t c, uint32_t stamp)
@@ -143,22 +166,37 @@ __device__ __forceinline__ bool warp_reserve_w(const WDev &d, uint32_t v, uint32
     return true;
 }
 
+__global__ void __launch_bounds__(256) w_heavy_flag_kernel(const uint32_t *off, uint32_t n, uint32_t *tail_stamp)
+{
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        tail_stamp[v] = off[v + 1] - off[v] >= WHEAVY_DEG ? WHEAVY_BIT : 0u;
+}
+
 // A head h of round lid - 1 whose smallest accepted root is mn: its
 // neighbours t > mn become tails of round lid (stamp lid), once each.  The
 // adjacency is in descending order, so the walk stops at the first t <= mn.
-// Called by one whole warp.
-__device__ __forceinline__ void w_mark_head(const WDev &d, uint32_t h, uint32_t mn, uint32_t lid, uint32_t *tails,
-                                            uint32_t *tails_cnt)
+// Called by whole warps; warp w of nw starts at chunk w.
+__device__ __forceinline__ void w_mark_head(const WDev &d, uint32_t h, uint32_t mn, uint32_t lid, const WTails &out,
+                                            uint32_t w = 0, uint32_t nw = 1)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t e_end = d.off[h + 1];
-    for (uint32_t e0 = d.off[h]; e0 < e_end; e0 += 32) {
+    for (uint32_t e0 = d.off[h] + 32 * w; e0 < e_end; e0 += 32 * nw) {
         const uint32_t e = e0 + lane;
         const bool in = e < e_end;
         const uint32_t t = in ? d.adj[e] : 0u;
         const bool ok = in && t > mn;
-        if (ok && d.tail_stamp[t] != lid) {
-            if (atomicExch(&d.tail_stamp[t], lid) != lid) tails[agg_append(tails_cnt)] = t;
+        const uint32_t ts = ok ? d.tail_stamp[t] : lid, mark = lid | (ts & WHEAVY_BIT);
+        if (ok && ts != mark && atomicExch(&d.tail_stamp[t], mark) != mark) {
+            if (!(ts & WHEAVY_BIT) || !out.heavy) {
+                out.light[agg_append(out.light_cnt)] = t;
+            } else {
+                const uint32_t slot = atomicAdd(out.heavy_cnt, 1u);
+                const uint32_t k = (d.off[t + 1] - d.off[t] + WITEM - 1) / WITEM;
+                const uint32_t at = atomicAdd(out.items_cnt, k);
+                out.heavy[slot] = t;
+                for (uint32_t j = 0; j < k; ++j) out.items[at + j] = make_uint2(slot, j);
+            }
         }
         if (__ballot_sync(FULL, in && !ok)) break;
     }
@@ -179,8 +217,8 @@ __device__ void w_rows_clear_phase(const WDev &d, uint32_t s)
 // front: the batch roots as the heads of the first round (host-driven loop);
 // with `tails` instead, the roots mark the first round's tails themselves.
 __device__ void w_root_init_phase(const WDev &d, uint32_t s, uint32_t nroots, uint32_t lid0, uint32_t *front,
-                                  uint32_t *front_cnt, uint32_t *news, uint32_t *news_cnt, uint32_t *tails = nullptr,
-                                  uint32_t *tails_cnt = nullptr)
+                                  uint32_t *front_cnt, uint32_t *news, uint32_t *news_cnt,
+                                  const WTails *tails = nullptr)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -208,7 +246,7 @@ __device__ void w_root_init_phase(const WDev &d, uint32_t s, uint32_t nroots, ui
             if (front) front[atomicAdd(front_cnt, 1u)] = r;
             news[atomicAdd(news_cnt, 1u)] = r;
         }
-        if (tails) w_mark_head(d, r, r, lid0 + 1, tails, tails_cnt);
+        if (tails) w_mark_head(d, r, r, lid0 + 1, *tails);
     }
 }
 
@@ -226,7 +264,7 @@ __device__ void w_mark_phase(const WDev &d, const uint32_t *front, uint32_t cnt,
     const int pp = (lid_cur - 1) & 1;
     for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < cnt; q += nw) {
         const uint32_t h = front[q];
-        w_mark_head(d, h, d.last_min[pp][h], lid_cur, tails, tails_cnt);
+        w_mark_head(d, h, d.last_min[pp][h], lid_cur, WTails{tails, tails_cnt});
     }
 }
 
@@ -287,16 +325,166 @@ __device__ __forceinline__ uint32_t cover_chunk(uint32_t pend, bool in, uint32_t
     return pend;
 }
 
+// Round minimum of the relaxations arriving at t over the adjacency entries
+// [e_begin, e_end), per root, in rmin (RMIN_EMPTY before); returns the number
+// of roots touched, listed in `touched`.  Short logs of active heads are
+// flattened into one item list over the lanes (inclusive counts sa), so one
+// round of loads covers 32 entries whichever heads they belong to; logs of 32
+// roots and more on average are walked head by head, without the search for
+// each item's head and with the touched roots listed at the end (a fifth of the
+// instructions per item; nearly all items of the first batch).
+template <bool FIRST>
+__device__ __forceinline__ uint32_t w_gather(const WDev &d, uint32_t t, uint32_t e_begin, uint32_t e_end, uint32_t s,
+                                             uint32_t lid_cur, int32_t *rmin, uint16_t *touched,
+                                             unsigned long long &bytes)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t below = (1u << lane) - 1u;
+    const int pp = (lid_cur - 1) & 1;
+    const uint32_t lid_prev = lid_cur - 1;
+    uint32_t ntouch = 0;
+    bool dense = false;
+    for (uint32_t e0 = e_begin; e0 < e_end; e0 += 32) {
+        const uint32_t e = e0 + lane;
+        const bool in = e < e_end;
+        const uint32_t h = in ? d.adj[e] : 0u;
+        const bool ge = in && h >= s;
+        // stamp, log position and size of every head: independent loads
+        const uint32_t st = ge ? d.act_stamp[pp][h] : 0u;
+        const uint64_t hp = ge ? d.last_pos[pp][h] : 0ull;
+        const uint32_t hc = ge ? d.last_cnt[pp][h] : 0u;
+        const bool act = ge && st == lid_prev;
+        const int32_t wt = act ? (int32_t)d.w[e] : 0;
+        const uint32_t ca = act ? hc : 0u;
+        const uint64_t pa = act ? hp : 0ull;
+        uint32_t sa = ca;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, sa, o);
+            if (lane >= o) sa += y;
+        }
+        const uint32_t tot = __shfl_sync(FULL, sa, 31);
+        uint32_t heads = __ballot_sync(FULL, act);
+        if (d.work)
+            bytes += __popc(__ballot_sync(FULL, in)) * 4ull + __popc(__ballot_sync(FULL, ge)) * 4ull +
+                     __popc(__ballot_sync(FULL, act)) * 13ull + 4ull * tot;
+        if (FIRST && tot >= 32u * __popc(heads) && tot) {
+            dense = true;
+            for (; heads; heads &= heads - 1) {
+                const int k = __ffs(heads) - 1;
+                const uint32_t *log = d.log[pp] + __shfl_sync(FULL, pa, k);
+                const uint32_t cnt = __shfl_sync(FULL, ca, k);
+                const int32_t ww = __shfl_sync(FULL, wt, k);
+#pragma unroll 4
+                for (uint32_t i = lane; i < cnt; i += 32) {
+                    const uint32_t x = log[i], cr = x >> 16;
+                    if (s + cr < t) atomicMin(&rmin[cr], (int32_t)(int16_t)((int32_t)(int16_t)(x & 0xffffu) + ww));
+                }
+            }
+            __syncwarp();
+            if (__ballot_sync(FULL, in && !ge)) break;
+            continue;
+        }
+        for (uint32_t i0 = 0; i0 < tot; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            uint32_t L = 0;  // head lane: the lanes whose inclusive count is <= i
+#pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(FULL, sa, L + step - 1) <= i) L += step;
+            const uint64_t qp = __shfl_sync(FULL, pa, L);
+            const uint32_t x0 = __shfl_sync(FULL, sa - ca, L);
+            const int32_t ww = __shfl_sync(FULL, wt, L);
+            bool fresh = false;
+            uint32_t cr = 0;
+            if (i < tot) {
+                const uint32_t x = d.log[pp][qp + (i - x0)];
+                cr = x >> 16;
+                if (s + cr < t) {
+                    const int32_t m = (int32_t)(int16_t)((int32_t)(int16_t)(x & 0xffffu) + ww);
+                    fresh = atomicMin(&rmin[cr], m) == RMIN_EMPTY;
+                }
+            }
+            // first touches of this round appended in lane order
+            const uint32_t fm = __ballot_sync(FULL, fresh);
+            if (fresh) touched[ntouch + __popc(fm & below)] = (uint16_t)cr;
+            ntouch += __popc(fm);
+        }
+        if (__ballot_sync(FULL, in && !ge)) break;
+    }
+    __syncwarp();
+    if (FIRST && dense) {
+        ntouch = 0;
+        for (uint32_t c0 = 0; c0 < d.B; c0 += 32) {
+            const uint32_t c = c0 + lane;
+            const bool have = c < d.B && rmin[c] != RMIN_EMPTY;
+            const uint32_t m = __ballot_sync(FULL, have);
+            if (have) touched[ntouch + __popc(m & below)] = (uint16_t)c;
+            ntouch += __popc(m);
+        }
+        __syncwarp();
+    }
+    return ntouch;
+}
+
+// The checks of one group of touched roots of t, one per lane (root c when
+// `have`, its round minimum in rmin): returns INT_MAX where the minimum is not
+// below dists_table, INT_MIN where it is accepted, else the value that covers it.
+template <bool FIRST>
+__device__ __forceinline__ int32_t w_check_group(const WDev &d, uint32_t t, bool have, uint32_t c, const int32_t *rmin,
+                                                 uint32_t s, uint32_t b, uint64_t cbase, uint32_t clen, uint32_t vql)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t B = d.B;
+    // checks (1) and (2) walk a list in order and stop at its first
+    // covering entry, as the reference's loops do.  The lanes hold 32
+    // consecutive entries of the list; the candidates still looking
+    // (bits of `pend`, one per lane of this group) are taken 4 at a
+    // time, each gathering its own row at the 32 entries' keys, and a
+    // ballot gives the first covering entry of each.  A candidate
+    // leaves the walk at the chunk that covers it.
+    int32_t m = 0, r = INT_MAX;
+    if (have) {
+        m = rmin[c];
+        if (m < dt_get(d, t, c, b + 1)) r = INT_MIN;  // accepted unless pruned below
+    }
+    uint32_t pend = __ballot_sync(FULL, r == INT_MIN);
+    // check (1): t's committed labels (hub, distance) against the
+    // candidate roots' dists_table rows (buf[c][hub])
+    for (uint32_t j0 = 0; j0 < clen && pend; j0 += 32) {
+        const bool in = j0 + lane < clen;
+        const uint32_t hl = in ? d.pool_hub[cbase + j0 + lane] : 0xffffffffu;
+        const int32_t dl = in ? (int32_t)d.pool_dist[cbase + j0 + lane] : 0;
+        pend = cover_chunk(pend, in, hl, hl, dl, d.buf, d.n, c, m, s, r);
+    }
+    // check (2) (batch 0 only): t's temporary labels in acceptance
+    // order (root, distance) against the snapshot rows of the
+    // candidates' temporary tables, roots before the candidate only
+    if (FIRST) {
+        const uint16_t *tqp = d.vq + (uint64_t)t * B;
+        const int16_t *trow = d.vd + (uint64_t)t * B;
+        for (uint32_t k0 = 0; k0 < vql && pend; k0 += 32) {
+            const bool in = k0 + lane < vql;
+            const uint32_t rl = in ? (uint32_t)tqp[k0 + lane] : 0u;
+            const int32_t tl = in ? (int32_t)trow[rl] : 0;
+            pend = cover_chunk(pend, in, rl, s + rl, tl, d.snap, B, c, m, s, r);
+        }
+    }
+    return r;
+}
+
 // The pull of one round (send_messages, pado_weighted_unv_unp.h:409-870, as
 // a pull).  Per-warp dynamic shared memory: rmin[B] int32, res[B] int32,
 // touched[B] u16.  Run by blocks of WPULL_WARPS warps.
 // tq: the round's work counter for dynamic tail claiming (null: static
-// grid-stride assignment).  front_next (may be null) collects the next round's
-// heads; next_tails (may be null) collects the next round's tails directly.
+// grid-stride assignment).  FIRST: batch 0, whose rounds are few, large and
+// need check (2) and the walk of long logs; the other batches' many small rounds
+// run a shorter instance.  front_next (may be null) collects the next round's
+// heads; next (may be null) collects the next round's tails directly.
+template <bool FIRST>
 __device__ void w_pull_phase(const WDev &d, const uint32_t *tails, uint32_t cnt, uint32_t s, uint32_t b,
                              uint32_t lid_cur, uint32_t *front_next, uint32_t *front_next_cnt, uint32_t *news,
                              uint32_t *news_cnt, uint32_t *retry, uint32_t *retry_cnt, unsigned char *wsm,
-                             uint32_t *tq = nullptr, uint32_t *next_tails = nullptr, uint32_t *next_tails_cnt = nullptr)
+                             uint32_t *tq = nullptr, const WTails *next = nullptr)
 {
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
@@ -306,71 +494,15 @@ __device__ void w_pull_phase(const WDev &d, const uint32_t *tails, uint32_t cnt,
     uint16_t *touched = reinterpret_cast<uint16_t *>(reinterpret_cast<int32_t *>(wsm) + (size_t)2 * WPULL_WARPS * B) +
                         (size_t)w * B;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    const int pp = (lid_cur - 1) & 1, cp = lid_cur & 1;
-    const uint32_t lid_prev = lid_cur - 1;
+    const int cp = lid_cur & 1;
     const uint32_t stamp = b + 1;
     for (uint32_t c = lane; c < B; c += 32) rmin[c] = RMIN_EMPTY;
     __syncwarp();
     unsigned long long bytes = 0;
-    const uint32_t below = (1u << lane) - 1u;
     auto pull_tail = [&](const uint32_t t) {
         bytes += 8;
-        // (a) round minimum of the relaxations arriving at t, per root.  The
-        // active heads' logged roots are flattened into one item list over
-        // the lanes (inclusive counts sa), so one round of loads covers 32
-        // entries whichever heads they belong to.
-        uint32_t ntouch = 0;  // roots touched so far, in `touched`
-        const uint32_t e_end = d.off[t + 1];
-        for (uint32_t e0 = d.off[t]; e0 < e_end; e0 += 32) {
-            const uint32_t e = e0 + lane;
-            const bool in = e < e_end;
-            const uint32_t h = in ? d.adj[e] : 0u;
-            const bool ge = in && h >= s;
-            // stamp, log position and size of every head: independent loads
-            const uint32_t st = ge ? d.act_stamp[pp][h] : 0u;
-            const uint64_t hp = ge ? d.last_pos[pp][h] : 0ull;
-            const uint32_t hc = ge ? d.last_cnt[pp][h] : 0u;
-            const bool act = ge && st == lid_prev;
-            const int32_t wt = act ? (int32_t)d.w[e] : 0;
-            const uint32_t ca = act ? hc : 0u;
-            const uint64_t pa = act ? hp : 0ull;
-            uint32_t sa = ca;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, sa, o);
-                if (lane >= o) sa += y;
-            }
-            const uint32_t tot = __shfl_sync(FULL, sa, 31);
-            if (d.work)
-                bytes += __popc(__ballot_sync(FULL, in)) * 4ull + __popc(__ballot_sync(FULL, ge)) * 4ull +
-                         __popc(__ballot_sync(FULL, act)) * 13ull + 4ull * tot;
-            for (uint32_t i0 = 0; i0 < tot; i0 += 32) {
-                const uint32_t i = i0 + lane;
-                uint32_t L = 0;  // head lane: the lanes whose inclusive count is <= i
-#pragma unroll
-                for (uint32_t step = 16; step > 0; step >>= 1)
-                    if (__shfl_sync(FULL, sa, L + step - 1) <= i) L += step;
-                const uint64_t qp = __shfl_sync(FULL, pa, L);
-                const uint32_t x0 = __shfl_sync(FULL, sa - ca, L);
-                const int32_t ww = __shfl_sync(FULL, wt, L);
-                bool fresh = false;
-                uint32_t cr = 0;
-                if (i < tot) {
-                    const uint32_t x = d.log[pp][qp + (i - x0)];
-                    cr = x >> 16;
-                    if (s + cr < t) {
-                        const int32_t m = (int32_t)(int16_t)((int32_t)(int16_t)(x & 0xffffu) + ww);
-                        fresh = atomicMin(&rmin[cr], m) == RMIN_EMPTY;
-                    }
-                }
-                // first touches of this round appended in lane order
-                const uint32_t fm = __ballot_sync(FULL, fresh);
-                if (fresh) touched[ntouch + __popc(fm & below)] = (uint16_t)cr;
-                ntouch += __popc(fm);
-            }
-            if (__ballot_sync(FULL, in && !ge)) break;
-        }
-        __syncwarp();
+        // (a) round minimum of the relaxations arriving at t, per root
+        const uint32_t ntouch = w_gather<FIRST>(d, t, d.off[t], d.off[t + 1], s, lid_cur, rmin, touched, bytes);
         if (ntouch == 0) return;
         // (b) candidates: round minimum below dists_table; checks (1) and (2)
         const uint64_t cbase = d.lab_off[t];
@@ -380,50 +512,13 @@ __device__ void w_pull_phase(const WDev &d, const uint32_t *tails, uint32_t cnt,
         for (uint32_t i0 = 0; i0 < ntouch; i0 += 32) {
             const uint32_t i = i0 + lane;
             bool acc = false, isnew = false;
-            // checks (1) and (2) walk a list in order and stop at its first
-            // covering entry, as the reference's loops do.  The lanes hold 32
-            // consecutive entries of the list; the candidates still looking
-            // (bits of `pend`, one per lane of this group) are taken 4 at a
-            // time, each gathering its own row at the 32 entries' keys, and a
-            // ballot gives the first covering entry of each.  A candidate
-            // leaves the walk at the chunk that covers it.
-            uint32_t c = 0, creal = 0;
-            int32_t m = 0, r = INT_MAX;  // INT_MAX: not a candidate
+            const uint32_t c = i < ntouch ? touched[i] : 0u;
+            const int32_t r = w_check_group<FIRST>(d, t, i < ntouch, c, rmin, s, b, cbase, clen, vql);
             if (i < ntouch) {
-                c = touched[i];
-                m = rmin[c];
-                creal = s + c;
-                if (m < dt_get(d, t, c, stamp)) r = INT_MIN;  // accepted unless pruned below
-            }
-            uint32_t pend = __ballot_sync(FULL, r == INT_MIN);
-            // check (1): t's committed labels (hub, distance) against the
-            // candidate roots' dists_table rows (buf[c][hub])
-            for (uint32_t j0 = 0; j0 < clen && pend; j0 += 32) {
-                const bool in = j0 + lane < clen;
-                const uint32_t hl = in ? d.pool_hub[cbase + j0 + lane] : 0xffffffffu;
-                const int32_t dl = in ? (int32_t)d.pool_dist[cbase + j0 + lane] : 0;
-                pend = cover_chunk(pend, in, hl, hl, dl, d.buf, d.n, c, m, s, r);
-            }
-            // check (2) (batch 0 only): t's temporary labels in acceptance
-            // order (root, distance) against the snapshot rows of the
-            // candidates' temporary tables, roots before the candidate only
-            if (b == 0) {
-                const uint16_t *tqp = d.vq + (uint64_t)t * B;
-                const int16_t *trow = d.vd + (uint64_t)t * B;
-                for (uint32_t k0 = 0; k0 < vql && pend; k0 += 32) {
-                    const bool in = k0 + lane < vql;
-                    const uint32_t rl = in ? (uint32_t)tqp[k0 + lane] : 0u;
-                    const int32_t tl = in ? (int32_t)trow[rl] : 0;
-                    pend = cover_chunk(pend, in, rl, s + rl, tl, d.snap, B, c, m, s, r);
-                }
-            }
-            if (i < ntouch) {
-                if (r != INT_MAX) {
-                    if (r == INT_MIN) {
-                        acc = true;
-                        isnew = d.vd[(uint64_t)t * B + c] == I16_INF;
-                        mnacc = min(mnacc, creal);
-                    }
+                if (r == INT_MIN) {
+                    acc = true;
+                    isnew = d.vd[(uint64_t)t * B + c] == I16_INF;
+                    mnacc = min(mnacc, s + c);
                 }
                 res[i] = r;
             }
@@ -495,9 +590,9 @@ __device__ void w_pull_phase(const WDev &d, const uint32_t *tails, uint32_t cnt,
             }
         }
         __syncwarp();
-        // t is a head of the next round: with next_tails it marks that
-        // round's tails itself (no separate mark phase)
-        if (nacc && next_tails) w_mark_head(d, t, mnacc, lid_cur + 1, next_tails, next_tails_cnt);
+        // t is a head of the next round: with `next` it marks that round's
+        // tails itself (no separate mark phase)
+        if (nacc && next) w_mark_head(d, t, mnacc, lid_cur + 1, *next);
     };
     if (tq) {
         for_claimed<0>(cnt, tq, [&](uint32_t q) { pull_tail(tails[q]); });
@@ -507,6 +602,147 @@ __device__ void w_pull_phase(const WDev &d, const uint32_t *tails, uint32_t cnt,
     if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_WPULL], bytes);
 }
 
+// The items of a round's heavy tails, a warp each: WITEM adjacency entries
+// min-reduced in shared memory, then into the tail's row of hmin.
+template <bool FIRST>
+__device__ __noinline__ void w_heavy_items_phase(const WDev &d, const WTails &tl, uint32_t nitems, uint32_t s, uint32_t lid_cur,
+                                    int32_t *hmin, uint32_t *claim, unsigned char *wsm)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t B = d.B;
+    int32_t *rmin = reinterpret_cast<int32_t *>(wsm) + (size_t)w * B;
+    uint16_t *touched = reinterpret_cast<uint16_t *>(reinterpret_cast<int32_t *>(wsm) + (size_t)2 * WPULL_WARPS * B) +
+                        (size_t)w * B;
+    for (uint32_t c = lane; c < B; c += 32) rmin[c] = RMIN_EMPTY;
+    __syncwarp();
+    unsigned long long bytes = 0;
+    for_claimed<0>(nitems, claim, [&](uint32_t q) {
+        const uint2 it = tl.items[q];
+        const uint32_t t = tl.heavy[it.x], e0 = d.off[t] + it.y * WITEM;
+        const uint32_t ntouch = w_gather<FIRST>(d, t, e0, min(e0 + WITEM, d.off[t + 1]), s, lid_cur, rmin, touched, bytes);
+        for (uint32_t i = lane; i < ntouch; i += 32) {
+            const uint32_t c = touched[i];
+            atomicMin(&hmin[(uint64_t)it.x * B + c], rmin[c]);
+            rmin[c] = RMIN_EMPTY;
+        }
+        __syncwarp();
+    });
+    if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_WPULL], bytes);
+}
+
+// The checks and commit of a round's heavy tails, a block each, once their
+// items are done: what pull_tail does from (b) on, the groups of 32 touched
+// roots spread over the block's warps.  Leaves the rows of hmin empty.
+template <bool FIRST>
+__device__ __noinline__ void w_heavy_finish_phase(const WDev &d, const uint32_t *heavy, uint32_t nheavy, uint32_t s, uint32_t b,
+                                     uint32_t lid_cur, uint32_t *news, uint32_t *news_cnt, uint32_t *retry,
+                                     uint32_t *retry_cnt, unsigned char *wsm, int32_t *hmin, const WTails &next)
+{
+    __shared__ uint32_t sum[5];  // touched, accepted, new, least accepted root, log room
+    __shared__ unsigned long long slpos;
+    __shared__ uint32_t gacc[MAX_BATCH / 32], gnew[MAX_BATCH / 32];  // per group: accepted and new lanes
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, cp = lid_cur & 1;
+    const uint32_t B = d.B, below = (1u << lane) - 1u;
+    int32_t *rmin = reinterpret_cast<int32_t *>(wsm);
+    int32_t *res = rmin + (size_t)WPULL_WARPS * B;
+    uint16_t *touched = reinterpret_cast<uint16_t *>(rmin + (size_t)2 * WPULL_WARPS * B);
+    for (uint32_t q = blockIdx.x; q < nheavy; q += gridDim.x) {
+        const uint32_t t = heavy[q];
+        int32_t *row = hmin + (uint64_t)q * B;
+        __syncthreads();  // the previous tail's shared state is done with
+        for (uint32_t c = threadIdx.x; c < B; c += WPULL_WARPS * 32) {
+            const int32_t x = __ldcg(row + c);
+            rmin[c] = x == HMIN_EMPTY ? RMIN_EMPTY : x;
+            if (x != HMIN_EMPTY) row[c] = HMIN_EMPTY;
+        }
+        if (threadIdx.x < 5) sum[threadIdx.x] = threadIdx.x == 3 ? 0xffffffffu : threadIdx.x == 4 ? 1u : 0u;
+        __syncthreads();
+        if (w == 0) {
+            uint32_t k = 0;
+            for (uint32_t c0 = 0; c0 < B; c0 += 32) {
+                const uint32_t c = c0 + lane;
+                const bool have = c < B && rmin[c] != RMIN_EMPTY;
+                const uint32_t m = __ballot_sync(FULL, have);
+                if (have) touched[k + __popc(m & below)] = (uint16_t)c;
+                k += __popc(m);
+            }
+            if (lane == 0) sum[0] = k;
+        }
+        __syncthreads();
+        const uint32_t ntouch = sum[0], ng = (ntouch + 31) / 32;
+        const uint64_t cbase = d.lab_off[t];
+        const uint32_t clen = d.lab_len[t], vql = d.vq_len[t];
+        for (uint32_t g = w; g < ng; g += WPULL_WARPS) {
+            const uint32_t i = g * 32 + lane;
+            const uint32_t c = i < ntouch ? touched[i] : 0u;
+            const int32_t r = w_check_group<FIRST>(d, t, i < ntouch, c, rmin, s, b, cbase, clen, vql);
+            if (i < ntouch) res[i] = r;
+            const bool acc = i < ntouch && r == INT_MIN;
+            const bool isnew = acc && d.vd[(uint64_t)t * B + c] == I16_INF;
+            const uint32_t am = __ballot_sync(FULL, acc), nm = __ballot_sync(FULL, isnew);
+            const uint32_t mn = warp_min_u32(acc ? s + c : 0xffffffffu);
+            if (lane == 0) {
+                gacc[g] = am;
+                gnew[g] = nm;
+                atomicAdd(&sum[1], (uint32_t)__popc(am));
+                atomicAdd(&sum[2], (uint32_t)__popc(nm));
+                atomicMin(&sum[3], mn);
+            }
+        }
+        __syncthreads();
+        const uint32_t nacc = sum[1], nnew = sum[2], mnacc = sum[3];
+        if (threadIdx.x == 0) {
+            if (d.work) atomicAdd(&d.work[W_WPULL], 8ull * ntouch + 12 + 6ull * clen * ntouch + 8ull * nacc);
+            if (nacc) {
+                slpos = atomicAdd(&d.log_top[cp], (unsigned long long)nacc);
+                if (slpos + nacc > d.log_cap) {  // re-run as a light tail after the log grows
+                    sum[4] = 0;
+                    atomicOr(d.status, ST_POOL_RETRY);
+                    retry[atomicAdd(retry_cnt, 1u)] = t;
+                }
+            }
+        }
+        __syncthreads();
+        if (!sum[4]) continue;  // uniform; nothing committed
+        const unsigned long long lpos = slpos;
+        for (uint32_t g = w; g < ng; g += WPULL_WARPS) {
+            // accepted and new roots of the groups before g
+            uint32_t accb = 0, newb = 0;
+            for (uint32_t j = lane; j < g; j += 32) {
+                accb += __popc(gacc[j]);
+                newb += __popc(gnew[j]);
+            }
+            accb = __reduce_add_sync(FULL, accb);
+            newb = __reduce_add_sync(FULL, newb);
+            const uint32_t i = g * 32 + lane;
+            if (i < ntouch) {
+                const uint32_t c = touched[i];
+                const int32_t m = rmin[c], r = res[i];
+                if (r != INT_MAX) dt_put(d, t, c, b + 1, r != INT_MIN && r < m ? r : m);
+                if (gacc[g] >> lane & 1u) {
+                    d.log[cp][lpos + accb + __popc(gacc[g] & below)] = (c << 16) | (uint32_t)(uint16_t)(int16_t)m;
+                    d.vd[(uint64_t)t * B + c] = (int16_t)m;
+                }
+                if (gnew[g] >> lane & 1u) d.vq[(uint64_t)t * B + vql + newb + __popc(gnew[g] & below)] = (uint16_t)c;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (nnew) {
+                d.vq_len[t] = vql + nnew;
+                if (vql == 0) news[atomicAdd(news_cnt, 1u)] = t;
+            }
+            if (nacc) {
+                d.last_pos[cp][t] = lpos;
+                d.last_cnt[cp][t] = nacc;
+                d.last_min[cp][t] = mnacc;
+                d.act_stamp[cp][t] = lid_cur;
+            }
+        }
+        if (nacc) w_mark_head(d, t, mnacc, lid_cur + 1, next, w, WPULL_WARPS);
+    }
+}
+
 __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_pull_kernel(WDev d, const uint32_t *tails, const uint32_t *tails_cnt,
                                                                   uint32_t s, uint32_t b, uint32_t lid_cur,
                                                                   uint32_t *front_next, uint32_t *front_next_cnt,
@@ -514,8 +750,12 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_pull_kernel(WDev d, con
                                                                   uint32_t *retry_cnt)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
-    w_pull_phase(d, tails, *tails_cnt, s, b, lid_cur, front_next, front_next_cnt, news, news_cnt, retry, retry_cnt,
-                 wsm);
+    if (b == 0)
+        w_pull_phase<true>(d, tails, *tails_cnt, s, b, lid_cur, front_next, front_next_cnt, news, news_cnt, retry,
+                           retry_cnt, wsm);
+    else
+        w_pull_phase<false>(d, tails, *tails_cnt, s, b, lid_cur, front_next, front_next_cnt, news, news_cnt, retry,
+                            retry_cnt, wsm);
 }
 
 // filter_out_labels (pado_weighted_unv_unp.h:1052-1184) on pre-filter values
@@ -602,21 +842,34 @@ __device__ __forceinline__ void w_commit_one(const WDev &d, uint32_t v, uint32_t
         }
         return;
     }
-    if (keep) {
-        for (uint32_t i0 = 0; i0 < L; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            const bool mine = i < L && !(vq[i] & 0x8000u);
-            const uint32_t key = mine ? vq[i] : 0xffffffffu;
-            uint32_t rank = 0;
-            for (uint32_t o0 = 0; o0 < L; o0 += 32) {
-                const uint32_t oj = o0 + lane;
-                const uint32_t other = (oj < L && !(vq[oj] & 0x8000u)) ? (uint32_t)vq[oj] : 0xffffffffu;
-                for (int k = 0; k < 32; ++k) rank += (__shfl_sync(FULL, other, k) < key) ? 1u : 0u;
+    if (keep && L <= 32) {
+        // one round: each root ranked by counting the smaller ones
+        const bool mine = (uint32_t)lane < L && !(vq[lane] & 0x8000u);
+        const uint32_t key = mine ? vq[lane] : 0xffffffffu;
+        uint32_t rank = 0;
+        for (uint32_t k = 0; k < L; ++k) rank += (__shfl_sync(FULL, key, k) < key) ? 1u : 0u;
+        if (mine) {
+            d.pool_hub[base + len + rank] = s + key;
+            d.pool_dist[base + len + rank] = row[key];
+        }
+    } else if (keep) {
+        // a bitmap of the batch's roots (B bits), read off in order
+        __shared__ uint32_t bitmaps[8][MAX_BATCH / 32];
+        uint32_t *bm = bitmaps[threadIdx.x >> 5];
+        for (uint32_t x = lane; x < (B + 31) / 32; x += 32) bm[x] = 0;
+        __syncwarp();
+        for (uint32_t i = lane; i < L; i += 32)
+            if (!(vq[i] & 0x8000u)) atomicOr(&bm[vq[i] >> 5], 1u << (vq[i] & 31));
+        __syncwarp();
+        uint64_t at = base + len;
+        for (uint32_t x = 0; x < (B + 31) / 32; ++x) {
+            const uint32_t m = bm[x];
+            if (m >> lane & 1u) {
+                const uint64_t o = at + __popc(m & ((1u << lane) - 1u));
+                d.pool_hub[o] = s + x * 32 + lane;
+                d.pool_dist[o] = row[x * 32 + lane];
             }
-            if (mine) {
-                d.pool_hub[base + len + rank] = s + key;
-                d.pool_dist[base + len + rank] = row[key];
-            }
+            at += __popc(m);
         }
     }
     __syncwarp();
@@ -748,26 +1001,34 @@ __global__ void __launch_bounds__(256) w_compact_kernel(WDev d, const uint64_t *
 enum WPhase : uint32_t { WP_START = 0, WP_ROUND = 1, WP_PULL_RETRY = 2, WP_END = 3, WP_COMMIT_RETRY = 4, WP_DONE = 5 };
 enum WExit : uint32_t { WX_RUNNING = 0, WX_DONE = 1, WX_NEED_LOG = 2, WX_NEED_POOL = 3, WX_STALL = 4 };
 
-// Round lid reads tails[lid % 3] and appends the next round's tails to
-// tails[(lid + 1) % 3] as its heads accept; the leader clears the third slot
-// for the round after.
+// Round lid reads slot lid % 3 of the tails and appends the next round's to
+// slot (lid + 1) % 3 as its heads accept; the leader clears the third slot for
+// the round after.
 struct WLoopCtl {
     GridBar bar;
     uint32_t phase, b, lid;           // resume point: phase, batch, last stamp
     uint32_t rounds, levels;
-    uint32_t tails_cnt[3], news_cnt[2];
-    uint32_t tq[3];                   // the pull's work counter, by the round's tails slot
+    uint32_t news_cnt[2];
+    struct Slot {                     // by round mod 3
+        uint32_t light_cnt, heavy_cnt, items_cnt;
+        uint32_t tq, iq;              // claims of light tails and of heavy tails' items
+    } slot[3];
     uint32_t heavy_cnt;               // batch 0's vertices with more than 32 temporary labels
     uint32_t rr_cnt, retry_cnt, status, exit_code;
 };
 
 struct WLoopBufs {
-    uint32_t *tails[3], *news[2];  // news by batch parity
+    uint32_t *tails[3], *htails[3], *news[2];  // news by batch parity
+    uint2 *items[3];
+    int32_t *hmin;                 // a row of B minima per heavy tail, HMIN_EMPTY between rounds
     uint32_t *rr, *retry, *heavy;
     uint32_t nbatches;
 };
 
-__global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLoopCtl *c, WLoopBufs bf)
+// The heavy phases are functions of their own (the parameters in constant
+// memory can be passed by reference): inlined, their registers made the many
+// small rounds spill (55.5 ms against 54.1 ms on wrmat18).
+__global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(const __grid_constant__ WDev d, WLoopCtl *c, const __grid_constant__ WLoopBufs bf)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
@@ -784,6 +1045,10 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
             c->exit_code = ex;
         }
     };
+    auto tails_of = [&](uint32_t x) {
+        WLoopCtl::Slot &t = c->slot[x];
+        return WTails{bf.tails[x], &t.light_cnt, bf.htails[x], &t.heavy_cnt, bf.items[x], &t.items_cnt};
+    };
     for (;;) {
         if (phase == WP_START) {
             if (b >= bf.nbatches) {
@@ -796,11 +1061,10 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
             // were cleared at the end of the previous batch; the roots mark
             // the first round's tails
             if (b > 0) w_rows_clear_phase(d, s - d.B);  // the previous batch's roots' temporary rows
-            w_root_init_phase(d, s, nr, lid0, nullptr, nullptr, bf.news[b & 1], &c->news_cnt[b & 1],
-                              bf.tails[(lid0 + 1) % 3], &c->tails_cnt[(lid0 + 1) % 3]);
+            const WTails first = tails_of((lid0 + 1) % 3);
+            w_root_init_phase(d, s, nr, lid0, nullptr, nullptr, bf.news[b & 1], &c->news_cnt[b & 1], &first);
             if (leader) {
-                c->tails_cnt[(lid0 + 2) % 3] = 0;  // filled by the first round
-                c->tq[(lid0 + 2) % 3] = 0;
+                c->slot[(lid0 + 2) % 3] = {};      // filled by the first round
                 d.log_top[(lid0 + 1) & 1] = 0;     // the first round's log
             }
             if (!sync.wait()) return;
@@ -824,12 +1088,22 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
                     if (!sync.wait()) return;
                 }
             }
-            w_pull_phase(d, bf.tails[tp], vload(&c->tails_cnt[tp]), s, b, lid_cur, nullptr, nullptr, bf.news[b & 1],
-                         &c->news_cnt[b & 1], bf.retry, &c->retry_cnt, wsm, &c->tq[tp], bf.tails[tn],
-                         &c->tails_cnt[tn]);
+            const WTails cur = tails_of(tp), next = tails_of(tn);
+            const uint32_t nheavy = vload(cur.heavy_cnt), nitems = vload(cur.items_cnt), nlight = vload(cur.light_cnt);
+            auto round = [&](auto first) {
+                constexpr bool FIRST = decltype(first)::value;
+                if (nheavy) w_heavy_items_phase<FIRST>(d, cur, nitems, s, lid_cur, bf.hmin, &c->slot[tp].iq, wsm);
+                w_pull_phase<FIRST>(d, cur.light, nlight, s, b, lid_cur, nullptr, nullptr, bf.news[b & 1],
+                                    &c->news_cnt[b & 1], bf.retry, &c->retry_cnt, wsm, &c->slot[tp].tq, &next);
+                if (!nheavy) return true;
+                if (!sync.wait()) return false;
+                w_heavy_finish_phase<FIRST>(d, cur.heavy, nheavy, s, b, lid_cur, bf.news[b & 1], &c->news_cnt[b & 1],
+                                            bf.retry, &c->retry_cnt, wsm, bf.hmin, next);
+                return true;
+            };
+            if (!(b == 0 ? round(std::true_type()) : round(std::false_type()))) return;
             if (leader) {
-                c->tails_cnt[(lid_cur + 2) % 3] = 0;  // read by the previous round's pull
-                c->tq[(lid_cur + 2) % 3] = 0;
+                c->slot[(lid_cur + 2) % 3] = {};      // read by the previous round's pull
                 d.log_top[(lid_cur + 1) & 1] = 0;     // the next round's log, last read by this pull
             }
             if (!sync.wait()) return;
@@ -840,7 +1114,7 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
             ++levels;
             ++rounds;
             lid = lid_cur;
-            phase = vload(&c->tails_cnt[tn]) ? WP_ROUND : WP_END;
+            phase = vload(next.light_cnt) + vload(next.heavy_cnt) ? WP_ROUND : WP_END;
             continue;
         }
         if (phase == WP_END || phase == WP_COMMIT_RETRY) {
@@ -850,8 +1124,7 @@ __global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(WDev d, WLo
                 if (leader) {
                     d.log_top[(lid + 1) & 1] = 0;  // the next batch's root log (read by the last pull)
                     c->news_cnt[nb ^ 1] = 0;       // the next batch's new-label list
-                    c->tails_cnt[(lid + 2) % 3] = 0;  // the next batch's first tails
-                    c->tq[(lid + 2) % 3] = 0;
+                    c->slot[(lid + 2) % 3] = {};   // the next batch's first tails
                 }
                 if (b == 0) {
                     // batch 0 has vertices with hundreds of temporary labels:
@@ -930,9 +1203,24 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     ws.add(rlen, B);
     ws.add(counters, 8);
     ws.add(snap, (uint64_t)B * B);
+    // at most m / WHEAVY_DEG vertices are heavy, with m / WITEM whole items and
+    // one partial each
+    const uint64_t hmax = std::min<uint64_t>(n, g.m / WHEAVY_DEG) + 1, imax = g.m / WITEM + hmax;
+    DBuf<int32_t> hmin;
+    DBuf<uint32_t> ht[3];
+    DBuf<uint2> hi[3];
+    ws.add(hmin, hmax * B);
+    for (int x = 0; x < 3; ++x) {
+        ws.add(ht[x], hmax);
+        ws.add(hi[x], imax);
+    }
     zeros.commit();
     ws.commit();
     zeros.mem.fill_bytes(0, s);
+    hmin.fill_bytes(0x7f, s);
+    if (n)
+        PADO_LAUNCH("w_heavy_flag_kernel", s,
+                    w_heavy_flag_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, tail_stamp.p));
     for (DBuf<int16_t> *t : {&buf, &vd})
         if (t->n)
             PADO_LAUNCH("w_fill_inf_kernel", s,
@@ -1032,7 +1320,8 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     try {
         PADO_CHECK(nbatches < 65535u, PADO_E_ARG, "more than 65534 batches");
         if (!host_loop && n) {
-            WLoopBufs bf{{tails.p, tails2.p, tails3.p}, {news.p, news2.p}, rr.p, retry.p, heavy.p, nbatches};
+            WLoopBufs bf{{tails.p, tails2.p, tails3.p}, {ht[0].p, ht[1].p, ht[2].p}, {news.p, news2.p},
+                         {hi[0].p, hi[1].p, hi[2].p}, hmin.p, rr.p, retry.p, heavy.p, nbatches};
             const void *kfn = (const void *)w_loop_kernel;
             PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pull_smem));
             int dev = 0, sms = 0, per_sm = 0;
@@ -1065,8 +1354,8 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
                     // the next round's tails marked so far stay
                     const uint32_t tp = (h.lid + 1) % 3;
                     PADO_CUDA(cudaMemcpyAsync(bf.tails[tp], retry.p, h.retry_cnt * 4ull, cudaMemcpyDeviceToDevice, s));
-                    h.tails_cnt[tp] = h.retry_cnt;
-                    h.tq[tp] = 0;  // the re-run pull claims from zero
+                    h.slot[tp] = {};  // the re-run pull claims from zero
+                    h.slot[tp].light_cnt = h.retry_cnt;
                 } else {
                     PADO_CHECK(h.exit_code == WX_NEED_POOL, PADO_E_STATE, "weighted labeling loop stopped unexpectedly");
                     unsigned long long top = 0;
