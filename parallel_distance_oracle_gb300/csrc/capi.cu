@@ -158,7 +158,7 @@ void label_into(pado_index *h, const pado::HostGraph &hg, const pado::DevGraph &
         h->bps.alloc(std::max<uint64_t>((uint64_t)n * K * 2, 1));
         pado::BpResult bp = pado::bp_label(hg, g, K, used, h->bpd.p, h->bps.p, s);
         phase("bit-parallel");
-        run = pado::unw_label(g, K, B, used, h->bpd.p, h->bps.p, h->store, s);
+        run = pado::unw_label(g, K, B, used, h->bpd.p, h->bps.p, pado::has_hubs(hg, 0, n), h->store, s);
         phase("labeling");
         h->info.bp_seconds = bp.ms * 1e-3;
         h->info.build_seconds = (bp.ms + run.ms) * 1e-3;
@@ -422,6 +422,15 @@ struct ManyRun {
     float bp_ms = 0.f;
     uint32_t bp_levels = 0;
 };
+
+// Whether most of the union's vertices are in graphs with hubs.
+bool mostly_hubs(const UnionGraph &u)
+{
+    uint64_t in = 0;
+    for (size_t i = 0; i + 1 < u.gbase.size(); ++i)
+        if (pado::has_hubs(u.hg, u.gbase[i], u.gbase[i + 1])) in += u.gbase[i + 1] - u.gbase[i];
+    return 2 * in > u.hg.n;
+}
 
 void many_bp(const UnionGraph &u, uint32_t K, ManyRun &r, cudaStream_t s)
 {
@@ -898,7 +907,8 @@ int pado_unw_build_many(uint32_t G, const uint32_t *n, const uint64_t *const *of
         many_bp(u, bp_roots, r, s);
         phase("bit-parallel");
         pado::LabelStore all;
-        pado::LabelRun run = pado::unw_label_many(r.g, u.gbase, bp_roots, batch, r.used, r.bpd.p, r.bps.p, all, s);
+        pado::LabelRun run = pado::unw_label_many(r.g, u.gbase, bp_roots, batch, r.used, r.bpd.p, r.bps.p,
+                                                  mostly_hubs(u), all, s);
         phase("labeling");
         // split: label totals at the graph boundaries, one upload of every
         // graph's ranks, then per graph its buffers, and ONE kernel copies
@@ -1000,7 +1010,7 @@ int pado_unw_tune_batch(uint32_t G, const uint32_t *n, const uint64_t *const *of
         for (uint32_t c = 0; c < ncand; ++c) {
             pado::LabelStore st;
             pado::LabelRun run = pado::unw_label_many(r.g, u.gbase, bp_roots, candidates[c], r.used, r.bpd.p, r.bps.p,
-                                                      st, s);
+                                                      mostly_hubs(u), st, s);
             if (ms) ms[c] = run.ms;
             if (c == 0 || run.ms < best_ms) {
                 best_ms = run.ms;

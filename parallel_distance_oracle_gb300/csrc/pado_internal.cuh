@@ -93,9 +93,20 @@ struct LabelRun {
     uint32_t batches = 0;
 };
 
-// unw.cu: batched pruned BFS labeling (pado_unw_unv_unp.h:425-1118).
+// Vertices of ids [lo, hi) that have hubs among them, judged by the first one
+// (the largest degree in a degree order): more than 8 times their average
+// degree.  R-MAT graphs lie above (16 times at 1,024 vertices, 2,000 at s20),
+// random graphs and grids with shortcuts below (3 and 2 times).  It only picks
+// the variant of the label loop that is faster on such graphs.
+inline bool has_hubs(const HostGraph &hg, uint32_t lo, uint32_t hi)
+{
+    return hi > lo && (uint64_t)(hg.off[lo + 1] - hg.off[lo]) * (hi - lo) > 8ull * (hg.off[hi] - hg.off[lo]);
+}
+
+// unw.cu: batched pruned BFS labeling (pado_unw_unv_unp.h:425-1118); hubs: see
+// has_hubs.
 LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<uint8_t> &used,
-                   const uint8_t *d_bpd, const uint64_t *d_bps, LabelStore &out, cudaStream_t s);
+                   const uint8_t *d_bpd, const uint64_t *d_bps, bool hubs, LabelStore &out, cudaStream_t s);
 
 // unw_many.cu: the same labeling for many independent graphs at once.  `g` is
 // the disjoint union, graph i owning ids [gbase[i], gbase[i+1]); every graph
@@ -103,7 +114,7 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
 // persistent launch.  `out` is indexed by union id with graph-local hubs.
 LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, uint32_t K, uint32_t B,
                         const std::vector<uint8_t> &used, const uint8_t *d_bpd, const uint64_t *d_bps,
-                        LabelStore &out, cudaStream_t s);
+                        bool hubs, LabelStore &out, cudaStream_t s);
 
 // weighted.cu: batched pruned relaxation (pado_weighted_unv_unp.h:281-1526).
 LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s);

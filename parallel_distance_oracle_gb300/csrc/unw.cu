@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) mark_kernel(UnwDev d, const uint32_t *fro
 __global__ void __launch_bounds__(PULL_THREADS, 4) pull_kernel(UnwDev d, PullArgs a)
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
-    pull_phase(d, a, pull_smem);
+    pull_phase<false>(d, a, pull_smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -168,6 +168,7 @@ __device__ void root_step_phase(const UnwDev &d, const uint32_t *roots, uint32_t
     if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_MARK], bytes);
 }
 
+template <bool LANES>
 __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, LoopCtl *c, LoopBufs bf)
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
@@ -242,7 +243,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, L
         a.dm = bf.dm[b & 1];
         a.tail_q = &c->tq[cur];
         a.htail_q = &c->hq[cur];
-        pull_phase(d, a, pull_smem);
+        pull_phase<LANES>(d, a, pull_smem);
         if (leader && phase == PH_LEVEL) {
             c->tcnt[(L + 2) % 3] = 0;
             c->hcnt[(L + 2) % 3] = 0;
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(UnwDev d, const uint64_t 
 }  // namespace
 
 LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<uint8_t> &used,
-                   const uint8_t *d_bpd, const uint64_t *d_bps, LabelStore &out, cudaStream_t s)
+                   const uint8_t *d_bpd, const uint64_t *d_bps, bool hubs, LabelStore &out, cudaStream_t s)
 {
     LabelRun run;
     const uint32_t n = g.n;
@@ -343,11 +344,12 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     zeros.add(counters, 8);
     zeros.add(status, 1);
     zeros.add(ctl, 1);
-    DBuf<uint8_t> d_used, bpmin;
+    DBuf<uint8_t> d_used, bpmin, bpdp;  // bpdp: only when rows of K bytes are not whole 16
     DBuf<uint32_t> last_min0, last_min1, ind, front0, front1, tails, htails, tails2, htails3, retry, roots, rr, d_broots,
         d_boff;
     ws.add(d_used, std::max<uint32_t>(n, 1));
     ws.add(bpmin, std::max<uint32_t>(n, 1));
+    ws.add(bpdp, K % 16 ? (uint64_t)n * ((K + 15) / 16 * 16) : 1);
     ws.add(last_min0, n);
     ws.add(last_min1, n);
     ws.add(ind, (uint64_t)n * words);
@@ -383,8 +385,12 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     d.used = d_used.p;
     d.bpd = d_bpd;
     d.bps = d_bps;
+    d.kp = (K + 15) / 16 * 16;
+    d.bpdp = d.kp == K ? d_bpd : bpdp.p;
     if (K && n)
-        PADO_LAUNCH("bpmin_kernel", s, bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p));
+        PADO_LAUNCH("bpmin_kernel", s,
+                    bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p, d.kp == K ? nullptr : bpdp.p,
+                                                                  d.kp));
     d.bpmin = bpmin.p;
     d.pool_hub = pool_hub.p;
     d.pool_dist = pool_dist.p;
@@ -473,7 +479,7 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
             LoopBufs bf{d_broots.p, d_boff.p, rr.p, {tails.p, front0.p, tails2.p}, {htails.p, front1.p, htails3.p},
                         retry.p, {dm.p, dm.p + (uint64_t)B * n}, trace ? bns.p : nullptr, trace ? llog.p : nullptr, level_cap,
                         nbatches};
-            const void *kfn = (const void *)label_loop_kernel;
+            const void *kfn = hubs ? (const void *)label_loop_kernel<false> : (const void *)label_loop_kernel<true>;
             PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int dev = 0, sms = 0, per_sm = 0;
             PADO_CUDA(cudaGetDevice(&dev));

@@ -58,6 +58,8 @@ struct UnwDev {
     const uint8_t *bpd;
     const uint64_t *bps;
     const uint8_t *bpmin;   // per vertex: least BP distance over the roots (255: none)
+    const uint8_t *bpdp;    // [n][kp]: bpd with rows of whole 16 bytes, 255 past K (bpd itself when K is such)
+    uint32_t kp;
     uint32_t *pool_hub;
     uint8_t *pool_dist;
     unsigned long long pool_cap;
@@ -111,12 +113,19 @@ __global__ void heavy_flag_kernel(const uint32_t *off, uint32_t n, uint8_t *flag
         if (off[v + 1] - off[v] >= HEAVY_DEG) flags[v] |= 2u;
 }
 
-// bpmin[v] = least BP distance of v over the K roots (255 if none reaches it).
-__global__ void bpmin_kernel(const uint8_t *bpd, uint32_t n, uint32_t K, uint8_t *bpmin)
+// bpmin[v] = least BP distance of v over the K roots (255 if none reaches it);
+// with bpdp, also the rows padded to kp bytes.
+__global__ void bpmin_kernel(const uint8_t *bpd, uint32_t n, uint32_t K, uint8_t *bpmin, uint8_t *bpdp, uint32_t kp)
 {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         uint32_t m = U8_INF;
-        for (uint32_t i = 0; i < K; ++i) m = min(m, (uint32_t)bpd[(uint64_t)v * K + i]);
+        for (uint32_t i = 0; i < K; ++i) {
+            const uint8_t x = bpd[(uint64_t)v * K + i];
+            m = min(m, (uint32_t)x);
+            if (bpdp) bpdp[(uint64_t)v * kp + i] = x;
+        }
+        if (bpdp)
+            for (uint32_t i = K; i < kp; ++i) bpdp[(uint64_t)v * kp + i] = U8_INF;
         bpmin[v] = (uint8_t)m;
     }
 }
@@ -416,6 +425,64 @@ __device__ __forceinline__ uint32_t bp_covered_group(const UnwDev &d, const uint
     for (int c = 0; c < BP_GROUP; ++c)
         if (__ballot_sync(FULL, cut(x0[c], s0[c], ts0) || cut(x1[c], s1[c], ts1))) res |= 1u << c;
     return res;
+}
+
+// The second BP stage with a lane per candidate, for groups of at least
+// BP_LANE_MIN: where tails have tens of candidates, a step per candidate makes
+// one tail's chain of loads decide the level.  Lane's root r (lanes in `need`)
+// against the tail's row in shared memory (`td`: distances, 255 for root 0 and
+// past K; `ts`: sets); returns whether the lane's candidate is covered and
+// leaves in `need` those to be tested a warp each.  All distances come in a few
+// 16-byte loads.  A sum x <= iter covers whatever the sets say and x > iter + 2
+// never does; the sets of the roots in between are read by the lane, two at a
+// time, when there are at most BP_LANE_OPEN per candidate (random graphs), and
+// left to the coalesced row loads of a warp otherwise (social graphs).  Sums
+// saturate at 255, so iter + 2 < 255 is required.
+constexpr uint32_t BP_LANE_MIN = 10, BP_LANE_OPEN = 12, BP_LANE_MAX_ITER = 250;
+__device__ __forceinline__ bool bp_covered_lanes(const UnwDev &d, uint32_t r, uint32_t &need, const uint32_t *td,
+                                                 const ulonglong2 *ts, uint32_t iter)
+{
+    const uint32_t lo4 = 0x02020202u, it4 = iter * 0x01010101u, one4 = it4 + 0x01010101u, hi4 = it4 + 0x02020202u;
+    const bool mine = need >> (threadIdx.x & 31) & 1u;
+    bool cov = false;
+    unsigned long long open = 0, first = 0;  // roots with x in (iter, iter + 2]; those with x = iter + 1
+    auto nibble = [](uint32_t m) { return (unsigned long long)(((m & 0x08040201u) * 0x01010101u) >> 24); };
+    const uint4 *row = reinterpret_cast<const uint4 *>(d.bpdp + (uint64_t)r * d.kp);
+    for (uint32_t q = 0; q < d.kp / 16; ++q) {
+        const uint4 v = mine ? row[q] : make_uint4(~0u, ~0u, ~0u, ~0u);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t x = __vaddus4(w[j], td[q * 4 + j]);
+            const uint32_t part = __vcmpgeu4(x, lo4) & __vcmpleu4(x, hi4), near = __vcmpleu4(x, it4);
+            cov = cov || (part & near);
+            open |= nibble(part & ~near) << (q * 16 + j * 4);
+            first |= nibble(__vcmpeq4(x, one4)) << (q * 16 + j * 4);
+        }
+    }
+    if (cov) open = 0;
+    need = __ballot_sync(FULL, open != 0);
+    if (!need || __reduce_add_sync(FULL, (uint32_t)__popcll(open)) > BP_LANE_OPEN * __popc(need)) return cov;
+    need = 0;
+    const ulonglong2 *rs = reinterpret_cast<const ulonglong2 *>(d.bps) + (uint64_t)r * d.K;
+    while (open) {
+        ulonglong2 a[2];
+        int i[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            i[u] = open ? __ffsll(open) - 1 : -1;
+            open &= open - 1;  // (0 stays 0)
+            a[u] = i[u] >= 0 ? rs[i[u]] : make_ulonglong2(0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const ulonglong2 t = ts[i[u] & 63];
+            cov = cov || (a[u].x & t.x) || ((first >> (i[u] & 63) & 1ull) && ((a[u].x & t.y) | (a[u].y & t.x)));
+        }
+        if (cov) break;
+    }
+    __syncwarp();
+    return cov;
 }
 
 struct PullArgs {
@@ -730,7 +797,9 @@ __device__ void pull_heavy_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
     if (tid == 0) UD_AT(d.ind_stamp, t, d.n, 1) = bc.b + 1;
 }
 
-// One light tail, processed by one warp.
+// One light tail, processed by one warp.  LANES: the second BP stage may take a
+// lane per candidate (see bp_covered_lanes).
+template <bool LANES>
 __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, WarpRegion &wr,
                                 unsigned long long &bytes)
 {
@@ -870,12 +939,26 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
             lane + 32 < (int)d.K ? UD_AT(reinterpret_cast<const ulonglong2 *>(d.bps), (uint64_t)t * d.K + lane + 32, (uint64_t)d.n * d.K, 3) : zero2;
         bytes += 17ull * (d.K - 1);
         uint32_t n2 = 0;
+        // t's row for a lane per candidate, in the bytes of the label stage
+        ulonglong2 *lts = reinterpret_cast<ulonglong2 *>(wr.sh);
+        uint32_t *ltd = wr.sh + MAX_BP * 4;
+        const bool lanes = LANES && iter <= BP_LANE_MAX_ITER && nsurv >= BP_LANE_MIN;
+        if (lanes) {
+            lts[lane] = ts0;
+            lts[lane + 32] = ts1;
+            reinterpret_cast<uint8_t *>(ltd)[lane] = lane ? td0 : (uint8_t)U8_INF;
+            reinterpret_cast<uint8_t *>(ltd)[lane + 32] = td1;
+            __syncwarp();
+        }
         for (uint32_t c0 = 0; c0 < nsurv; c0 += 32) {
             const uint32_t c = c0 + lane;
             const bool in = c < nsurv;
             const uint16_t ent = in ? wr.offered[c] : (uint16_t)0;
             uint32_t need = __ballot_sync(FULL, in && !(ent & 0x8000u));
             bool covered = false;
+            if (lanes && __popc(need) >= (int)BP_LANE_MIN) {
+                covered = bp_covered_lanes(d, s + (ent & 0x7fffu), need, ltd, lts, iter);
+            }
             while (need) {
                 int kk[BP_GROUP];
                 uint32_t rg[BP_GROUP], nc = 0;
@@ -1055,6 +1138,7 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
 
 // Pull phase of a level: heavy tails block-by-block, then light tails
 // warp-by-warp.  Ends with the block converged.
+template <bool LANES>
 __device__ void pull_phase(const UnwDev &d, const PullArgs &a, unsigned char *pull_smem)
 {
     const int lane = threadIdx.x & 31;
@@ -1097,11 +1181,11 @@ __device__ void pull_phase(const UnwDev &d, const PullArgs &a, unsigned char *pu
     }
     WarpRegion wr = warp_region(pull_smem, d.words, d.B, threadIdx.x >> 5);
     if (a.tail_q) {
-        for_claimed<0>(cnt, a.tail_q, [&](uint32_t q) { pull_light_tail(d, a, a.tails[q], wr, bytes); });
+        for_claimed<0>(cnt, a.tail_q, [&](uint32_t q) { pull_light_tail<LANES>(d, a, a.tails[q], wr, bytes); });
     } else {
         const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
         for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < cnt; q += nw)
-            pull_light_tail(d, a, a.tails[q], wr, bytes);
+            pull_light_tail<LANES>(d, a, a.tails[q], wr, bytes);
     }
     if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_PULL], bytes);
     __syncthreads();

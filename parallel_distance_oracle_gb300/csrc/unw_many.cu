@@ -172,6 +172,7 @@ __device__ void many_bookkeep(const UnwDev &d, ManyCtl *c, const ManyBufs &bf, u
     }
 }
 
+template <bool LANES>
 __global__ void __launch_bounds__(PULL_THREADS, 4) many_loop_kernel(UnwDev d, ManyCtl *c, ManyBufs bf)
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) many_loop_kernel(UnwDev d, Ma
         } else {
             many_root_step(d, bf, c, bf.rr, vload(&c->rr_cnt), L);
         }
-        pull_phase(d, a, pull_smem);
+        pull_phase<LANES>(d, a, pull_smem);
         if (leader) {
             c->tcnt[(L + 2) % 3] = 0;
             c->hcnt[(L + 2) % 3] = 0;
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(256) many_finalize_kernel(UnwDev d, const uint
 
 LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, uint32_t K, uint32_t B,
                         const std::vector<uint8_t> &used, const uint8_t *d_bpd, const uint64_t *d_bps,
-                        LabelStore &out, cudaStream_t s)
+                        bool hubs, LabelStore &out, cudaStream_t s)
 {
     LabelRun run;
     const uint32_t n = g.n;
@@ -325,7 +326,7 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     zeros.add(last1, n);
     for (DBuf<uint32_t> *x : {&lab_len, &lab_cap, &tail_stamp, &ind_stamp}) zeros.add(*x, n);
     zeros.add(status, 1);
-    DBuf<uint8_t> d_used, bpmin;
+    DBuf<uint8_t> d_used, bpmin, bpdp;  // bpdp: only when rows of K bytes are not whole 16
     DBuf<uint32_t> last_min0, last_min1, ind, tl0, tl1, tl2, th0, th1, th2, rretry, tretry, rq0b, rq1b, zq0b, zq1b, rr;
     DBuf<uint32_t> d_broots, d_bcnt, d_gbase;
     DBuf<GDesc> d_gd;
@@ -333,6 +334,7 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     DBuf<ManyCtl> ctl;
     ws.add(d_used, std::max<uint32_t>(n, 1));
     ws.add(bpmin, std::max<uint32_t>(n, 1));
+    ws.add(bpdp, K % 16 ? (uint64_t)n * ((K + 15) / 16 * 16) : 1);
     ws.add(ind, (uint64_t)n * words);
     for (DBuf<uint32_t> *x : {&last_min0, &last_min1, &tl0, &tl1, &tl2, &th0, &th1, &th2, &rretry, &tretry, &rq0b, &rq1b,
                               &zq0b, &zq1b, &rr})
@@ -379,8 +381,12 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     d.used = d_used.p;
     d.bpd = d_bpd;
     d.bps = d_bps;
+    d.kp = (K + 15) / 16 * 16;
+    d.bpdp = d.kp == K ? d_bpd : bpdp.p;
     if (K && n)
-        PADO_LAUNCH("bpmin_kernel", s, bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p));
+        PADO_LAUNCH("bpmin_kernel", s,
+                    bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p, d.kp == K ? nullptr : bpdp.p,
+                                                                  d.kp));
     d.bpmin = bpmin.p;
     d.pool_hub = pool_hub.p;
     d.pool_dist = pool_dist.p;
@@ -426,7 +432,7 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     PADO_CUDA(cudaEventRecord(e0, s));
     try {
         if (active) {
-            const void *kfn = (const void *)many_loop_kernel;
+            const void *kfn = hubs ? (const void *)many_loop_kernel<false> : (const void *)many_loop_kernel<true>;
             PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int dev = 0, sms = 0, per_sm = 0;
             PADO_CUDA(cudaGetDevice(&dev));
