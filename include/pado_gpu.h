@@ -209,11 +209,11 @@ int pado_reduce_equivalent_device(uint64_t m, const uint32_t *d_u, const uint32_
  * bytes per edge) from a memory pool of the library's own, in stream order.
  * Up to `bytes` of it stay reserved on the current device between calls
  * (default 0: every ingest call returns its scratch); a service that ingests
- * graphs repeatedly keeps them to skip the device allocations.  pado_query
- * takes its device buffer from the same pool and leaves at most the larger of
- * `bytes` and 32 MiB reserved; its calls of up to 16,384 pairs use page-locked
- * slots instead (160 KB each, at most eight kept).  Setting 0 releases what is
- * kept, the slots included. */
+ * graphs repeatedly keeps them to skip the device allocations.  pado_query and
+ * pado_export take device buffers from the same pool and leave at most the
+ * larger of `bytes` and 32 MiB reserved; pado_query's calls of up to 16,384
+ * pairs use page-locked slots instead (160 KB each, at most eight kept).
+ * Setting 0 releases what is kept, the slots included. */
 int pado_set_scratch_cache(uint64_t bytes);
 
 /* Ingest + labeling in one call, the graph staying on the device between

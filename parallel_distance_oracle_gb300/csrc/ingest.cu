@@ -214,34 +214,6 @@ cudaMemPool_t scratch_pool()
 
 namespace {
 
-template <typename T>
-struct PBuf {
-    T *p = nullptr;
-    size_t n = 0;
-    cudaStream_t s = nullptr;
-    PBuf(size_t count, cudaStream_t st) : n(count), s(st)
-    {
-        if (count) {
-            alloc_point();
-            PADO_CUDA(cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), scratch_pool(), s));
-            alloc_live(1);
-        }
-    }
-    PBuf(const PBuf &) = delete;
-    PBuf &operator=(const PBuf &) = delete;
-    ~PBuf()
-    {
-        if (p) {
-            cudaFreeAsync(p, s);
-            alloc_live(-1);
-        }
-    }
-    void zero()
-    {
-        if (n) PADO_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
-    }
-};
-
 // ---- radix sort -------------------------------------------------------------
 
 // The keys are split into `gridDim.x` runs of `per` whole tiles, a block
@@ -1103,6 +1075,24 @@ IngestResult ingest_edges(uint64_t m, const uint32_t *du, const uint32_t *dv, co
 void release_scratch(uint64_t keep_bytes)
 {
     PADO_CUDA(cudaMemPoolTrimTo(scratch_pool(), keep_bytes));
+}
+
+// Vertex v's share of an export in original-id order: the length of the list of
+// its rank; entry n closes the scan.
+__global__ void __launch_bounds__(256) export_len_kernel(const uint32_t *rank, const uint64_t *roff, uint32_t n,
+                                                         uint32_t *len)
+{
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
+        len[v] = v < n ? (uint32_t)(roff[rank[v] + 1] - roff[rank[v]]) : 0u;
+}
+
+void export_offsets(uint32_t n, const uint32_t *rank, const uint64_t *roff, uint64_t *noff, cudaStream_t s)
+{
+    PBuf<uint32_t> len((uint64_t)n + 1, s), sums(scan_sums_needed((uint64_t)n + 1), s);
+    PADO_LAUNCH("export_len_kernel", s,
+                export_len_kernel<<<grid_for((uint64_t)n + 1, 256), 256, 0, s>>>(rank, roff, n, len.p));
+    exclusive_scan(len.p, (uint64_t)n + 1, sums.p, s);
+    widen_u32(len.p, (uint64_t)n + 1, noff, s);
 }
 
 void widen_u32(const uint32_t *a, uint64_t n, uint64_t *b, cudaStream_t s)

@@ -160,8 +160,39 @@ ReduceResult reduce_equivalent(uint64_t m, const uint32_t *du, const uint32_t *d
 
 // The current device's scratch pool (ingest.cu), for stream-ordered buffers.
 cudaMemPool_t scratch_pool();
+// A buffer from it, freed in stream order.
+template <typename T>
+struct PBuf {
+    T *p = nullptr;
+    size_t n = 0;
+    cudaStream_t s = nullptr;
+    PBuf(size_t count, cudaStream_t st) : n(count), s(st)
+    {
+        if (count) {
+            alloc_point();
+            PADO_CUDA(cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), scratch_pool(), s));
+            alloc_live(1);
+        }
+    }
+    PBuf(const PBuf &) = delete;
+    PBuf &operator=(const PBuf &) = delete;
+    ~PBuf()
+    {
+        if (p) {
+            cudaFreeAsync(p, s);
+            alloc_live(-1);
+        }
+    }
+    void zero()
+    {
+        if (n) PADO_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
+    }
+};
 // Trims the scratch pool of the current device to keep_bytes.
 void release_scratch(uint64_t keep_bytes);
+// Offsets of an export in original-id order (device, n + 1): the lists of
+// rank[v], fewer than 2^32 entries in all.
+void export_offsets(uint32_t n, const uint32_t *rank, const uint64_t *roff, uint64_t *noff, cudaStream_t s);
 // b[i] = a[i] for i < n (device arrays, stream-ordered).
 void widen_u32(const uint32_t *a, uint64_t n, uint64_t *b, cudaStream_t s);
 
