@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) mark_kernel(UnwDev d, const uint32_t *fro
 __global__ void __launch_bounds__(PULL_THREADS, 4) pull_kernel(UnwDev d, PullArgs a)
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
-    pull_phase<false>(d, a, pull_smem);
+    pull_phase<0>(d, a, pull_smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -128,6 +128,7 @@ struct LoopBufs {
 };
 
 // Batch step for roots[0, nr): self label at stamp L, dist_matrix row, tails for L+1.
+template <int MODE>
 __device__ void root_step_phase(const UnwDev &d, const uint32_t *roots, uint32_t nr, uint32_t s, uint32_t b,
                                 uint32_t L, uint8_t *dm, const LoopBufs &bf, LoopCtl *c)
 {
@@ -161,6 +162,12 @@ __device__ void root_step_phase(const UnwDev &d, const uint32_t *roots, uint32_t
         __syncwarp();
         // dist_matrix row of r from all its labels, the new (r, 0) included
         uint8_t *row = dm + (uint64_t)idx * d.n;
+        if (MODE == 2) {  // the older labels are in already (rows_phase)
+            if (lane == 0) {
+                UD_AT(row, r, d.n, 4) = 0;
+                bm_set(d.bm + (b & 1) * bm_words(d.n, d.words), d.words, r, idx, 0);
+            }
+        } else
         for (uint32_t j = lane; j <= len; j += 32)
             UD_AT(row, UD_AT(d.pool_hub, base + j, d.pool_cap, 2), d.n, 4) = UD_AT(d.pool_dist, base + j, d.pool_cap, 2);
         mark_tails(d, r, r, L + 1, bf.tails[nx], &c->tcnt[nx], bf.htails[nx], &c->hcnt[nx], lane, 0, 1, bytes);
@@ -168,7 +175,7 @@ __device__ void root_step_phase(const UnwDev &d, const uint32_t *roots, uint32_t
     if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_MARK], bytes);
 }
 
-template <bool LANES>
+template <int MODE>
 __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, LoopCtl *c, LoopBufs bf)
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
@@ -184,13 +191,20 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, L
             const uint32_t s = b * d.B;
             uint8_t *dm = bf.dm[b & 1];
             if (phase == PH_BATCH) {
-                // rows of the previous batch go back to 255 (other parity)
-                if (b > 0)
+                if (MODE == 2) {
+                    if (b > 0)
+                        rows_phase(d, bf.broots + bf.boff[b - 1], bf.boff[b] - bf.boff[b - 1], s - d.B, bf.dm[(b - 1) & 1],
+                                   d.bm + ((b - 1) & 1) * bm_words(d.n, d.words), false);
+                    rows_phase(d, bf.broots + bf.boff[b], bf.boff[b + 1] - bf.boff[b], s, dm,
+                               d.bm + (b & 1) * bm_words(d.n, d.words), true);
+                    if (!sync.wait()) return;  // the root step moves and extends the lists
+                } else if (b > 0)
+                    // rows of the previous batch go back to 255 (other parity)
                     dm_rows_phase(d, bf.broots + bf.boff[b - 1], bf.boff[b] - bf.boff[b - 1], s - d.B, 0,
                                   nullptr, nullptr, bf.dm[(b - 1) & 1]);
-                root_step_phase(d, bf.broots + bf.boff[b], bf.boff[b + 1] - bf.boff[b], s, b, L, dm, bf, c);
+                root_step_phase<MODE>(d, bf.broots + bf.boff[b], bf.boff[b + 1] - bf.boff[b], s, b, L, dm, bf, c);
             } else {
-                root_step_phase(d, bf.rr, vload(&c->rr_cnt), s, b, L, dm, bf, c);
+                root_step_phase<MODE>(d, bf.rr, vload(&c->rr_cnt), s, b, L, dm, bf, c);
             }
             if (leader) {
                 c->tcnt[(L + 2) % 3] = 0;
@@ -241,9 +255,10 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) label_loop_kernel(UnwDev d, L
         a.next_htails_cnt = &c->hcnt[nx];
         a.next_stamp = L + 1;
         a.dm = bf.dm[b & 1];
+        if (MODE == 2) a.bm = d.bm + (b & 1) * bm_words(d.n, d.words);
         a.tail_q = &c->tq[cur];
         a.htail_q = &c->hq[cur];
-        pull_phase<LANES>(d, a, pull_smem);
+        pull_phase<MODE>(d, a, pull_smem);
         if (leader && phase == PH_LEVEL) {
             c->tcnt[(L + 2) % 3] = 0;
             c->hcnt[(L + 2) % 3] = 0;
@@ -311,7 +326,7 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     const char *loop_env = std::getenv("PADO_LEVEL_LOOP");
     const bool host_loop = loop_env && !strcmp(loop_env, "host");
     const uint32_t nbatches = (uint32_t)(((uint64_t)n + B - 1) / B);
-    uint64_t cap = initial_pool_entries(n);
+    uint64_t cap = initial_pool_entries(n, hubs);
     // one allocation that starts as zeros, one whose contents do not matter,
     // and, unless they are small, the label pool and dist_matrix (255s; a
     // second buffer for odd batches in the persistent loop) apart
@@ -369,7 +384,14 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     d_used.upload(used.data(), n, s);
     if (n) PADO_LAUNCH("heavy_flag_kernel", s, heavy_flag_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, d_used.p));
 
+    DBuf<uint32_t> bm;
+    if (!hubs && !host_loop && bm_shape(words) && 2 * bm_words(n, words) * 4 <= BM_MAX_BYTES) {
+        bm.alloc(2 * bm_words(n, words));
+        bm.fill_bytes(0, s);
+    }
+
     UnwDev d{};
+    d.bm = bm.p;
     d.n = n;
     d.K = K;
     d.B = B;
@@ -479,7 +501,9 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
             LoopBufs bf{d_broots.p, d_boff.p, rr.p, {tails.p, front0.p, tails2.p}, {htails.p, front1.p, htails3.p},
                         retry.p, {dm.p, dm.p + (uint64_t)B * n}, trace ? bns.p : nullptr, trace ? llog.p : nullptr, level_cap,
                         nbatches};
-            const void *kfn = hubs ? (const void *)label_loop_kernel<false> : (const void *)label_loop_kernel<true>;
+            const void *kfn = hubs    ? (const void *)label_loop_kernel<0>
+                              : !bm.n ? (const void *)label_loop_kernel<1>
+                                      : (const void *)label_loop_kernel<2>;
             PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int dev = 0, sms = 0, per_sm = 0;
             PADO_CUDA(cudaGetDevice(&dev));

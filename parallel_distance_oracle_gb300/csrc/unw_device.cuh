@@ -73,6 +73,7 @@ struct UnwDev {
     uint32_t *ind;        // n * words
     uint32_t *ind_stamp;  // batch + 1 when the row is valid
     uint8_t *dm;          // B * n
+    uint32_t *bm;         // cover bitmaps, two by batch parity (null: none), see BmShape
     uint32_t *status;
     unsigned long long *work;  // algorithmic-byte counters (profiling only)
 };
@@ -207,6 +208,65 @@ __device__ void root_init_phase(const UnwDev &d, const uint32_t *roots, uint32_t
     }
 }
 
+// Cover bitmaps of a batch (graphs without hubs): for every hub h and slack
+// 1 <= e <= BM_SLACKS, a bit per root of the batch: set when the root's
+// distance to h is at most e.  Row (h, e) is at (h * BM_SLACKS + e - 1) * words.
+// One 16-byte load then tells which of 128 candidates a label of slack e covers,
+// where dist_matrix is gathered a byte per candidate and label.  Filled from the
+// roots' labels like dist_matrix and cleared with it.  Used while they fit half
+// of L2 (beyond it their misses cost more than the gathers: 64 graphs of 4,400
+// vertices, 573 MB, 30.4 -> 36.5 ms; a random graph of 20,011 vertices, B = 512,
+// 20 MB, 17.1 -> 14.8 ms of label loop).
+constexpr uint32_t BM_SLACKS = 8;
+constexpr uint64_t BM_MAX_BYTES = 64ull << 20;  // both parities: half of L2
+constexpr int BM_LOADS = 4;
+__host__ __device__ __forceinline__ uint64_t bm_words(uint32_t n, uint32_t words)
+{
+    return (uint64_t)n * BM_SLACKS * words;
+}
+// Whether batches of `words` words split into whole 16-byte loads of a power of two of lanes.
+__host__ __device__ __forceinline__ bool bm_shape(uint32_t words)
+{
+    return words >= 4 && words <= 128 && (words & (words - 1)) == 0;
+}
+__device__ __forceinline__ void bm_set(uint32_t *bm, uint32_t words, uint32_t h, uint32_t idx, uint32_t dist)
+{
+    uint32_t *row = bm + (uint64_t)h * BM_SLACKS * words + (idx >> 5);
+    for (uint32_t e = max(dist, 1u); e <= BM_SLACKS; ++e) atomicOr(row + (e - 1) * words, 1u << (idx & 31));
+}
+// Clears the word that holds root idx (the others in it end with the same batch).
+__device__ __forceinline__ void bm_clear(uint32_t *bm, uint32_t words, uint32_t h, uint32_t idx, uint32_t dist)
+{
+    uint32_t *row = bm + (uint64_t)h * BM_SLACKS * words + (idx >> 5);
+    for (uint32_t e = max(dist, 1u); e <= BM_SLACKS; ++e) row[(e - 1) * words] = 0u;
+}
+
+// dist_matrix rows and cover bitmaps of a batch's roots from their labels (fill)
+// or back to 255 and 0, ROW_PARTS warps per root: the lists are long where
+// bitmaps are used, and a warp per root made a batch's start 88 us longer.
+constexpr uint32_t ROW_PARTS = 8;
+__device__ void rows_phase(const UnwDev &d, const uint32_t *roots, uint32_t nroots, uint32_t s, uint8_t *dm, uint32_t *bm,
+                           bool fill)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < nroots * ROW_PARTS; q += nw) {
+        const uint32_t r = roots[q / ROW_PARTS], idx = r - s;
+        const uint64_t base = UD_AT(d.lab_off, r, d.n, 1);
+        const uint32_t len = UD_AT(d.lab_len, r, d.n, 1);
+        uint8_t *row = dm + (uint64_t)idx * d.n;
+        for (uint32_t j = q % ROW_PARTS * 32 + lane; j < len; j += ROW_PARTS * 32) {
+            const uint32_t h = UD_AT(d.pool_hub, base + j, d.pool_cap, 2);
+            const uint8_t dd = UD_AT(d.pool_dist, base + j, d.pool_cap, 2);
+            UD_AT(row, h, d.n, 4) = fill ? dd : (uint8_t)U8_INF;
+            if (fill)
+                bm_set(bm, d.words, h, idx, dd);
+            else
+                bm_clear(bm, d.words, h, idx, dd);
+        }
+    }
+}
+
 // dist_matrix rows of the batch roots: fill from their labels (value = d) or
 // reset to 255 (pado_unw_unv_unp.h:492-526 and :780-816).
 // With gmap set, root r's row is (r - base) % B of its graph's block (batches
@@ -292,6 +352,8 @@ struct WarpRegion {
     uint32_t *sh;         // SMALL_CAP
     uint8_t *sd;          // SMALL_CAP
     uint32_t *ctr;        // spare
+    // with cover bitmaps the stage's last entries hold the candidates not covered yet
+    __device__ __forceinline__ uint32_t *open() const { return sh + SMALL_CAP - MAX_BATCH / 32; }
 };
 
 __host__ __device__ __forceinline__ uint32_t warp_region_bytes(uint32_t words, uint32_t B)
@@ -505,6 +567,7 @@ struct PullArgs {
     uint32_t *next_htails = nullptr, *next_htails_cnt = nullptr;
     uint32_t next_stamp = 0;
     uint8_t *dm = nullptr;           // dist_matrix of the current batch (default d.dm)
+    uint32_t *bm = nullptr;          // cover bitmaps of the current batch
     // Work counters for dynamic assignment (zero at the start of the level):
     // warps / blocks claim the next light / heavy tail from them, so that the
     // level ends when the work runs out rather than when the unluckiest
@@ -517,17 +580,18 @@ struct PullArgs {
 struct BatchCtx {
     uint32_t s, e, b, iter, base, dn;
     uint8_t *dm;
+    uint32_t *bm;
     uint32_t g;
 };
 
 __device__ __forceinline__ BatchCtx tail_ctx(const UnwDev &d, const PullArgs &a, uint32_t t)
 {
-    if (!a.gmap) return BatchCtx{a.s, a.e_roots, a.b, a.iter, 0u, d.n, a.dm ? a.dm : d.dm, 0u};
+    if (!a.gmap) return BatchCtx{a.s, a.e_roots, a.b, a.iter, 0u, d.n, a.dm ? a.dm : d.dm, a.bm, 0u};
     const uint32_t g = a.gmap[t];
     const GDesc &x = a.gd[g];
     return BatchCtx{gd_u32(x.s),    gd_u32(x.e), gd_u32(x.b),
                     gd_u32(x.iter), x.base,      x.n,
-                    d.dm + x.dm_off + (uint64_t)gd_u32(x.dmp) * d.B * x.n, g};
+                    d.dm + x.dm_off + (uint64_t)gd_u32(x.dmp) * d.B * x.n, nullptr, g};
 }
 
 // Marks the tails of head h for the level stamped `stamp`: neighbours t > mn
@@ -569,6 +633,7 @@ __device__ __forceinline__ void mark_tails(const UnwDev &d, uint32_t h, uint32_t
 }
 
 // One heavy tail, processed by the whole block.
+template <int MODE>
 __device__ void pull_heavy_tail(const UnwDev &d, const PullArgs &a, uint32_t t, HeavyRegion &hs,
                                 unsigned long long &bytes)
 {
@@ -773,6 +838,7 @@ __device__ void pull_heavy_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
             UD_AT(d.pool_hub, nbase + len + j, d.pool_cap, 2) = s + idx;
             UD_AT(d.pool_dist, nbase + len + j, d.pool_cap, 2) = (uint8_t)iter;
             if (is_root) UD_AT(bc.dm, (uint64_t)(t - s) * bc.dn + (s + idx - bc.base), (uint64_t)d.B * bc.dn, 4) = (uint8_t)iter;
+            if (MODE == 2 && is_root) bm_set(bc.bm, d.words, s + idx, t - s, iter);
             atomicMin(&hs.ctr[4], s + idx);
         }
         __syncthreads();
@@ -797,9 +863,10 @@ __device__ void pull_heavy_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
     if (tid == 0) UD_AT(d.ind_stamp, t, d.n, 1) = bc.b + 1;
 }
 
-// One light tail, processed by one warp.  LANES: the second BP stage may take a
-// lane per candidate (see bp_covered_lanes).
-template <bool LANES>
+// One light tail, processed by one warp.  MODE 1 and up: the second BP stage
+// may take a lane per candidate (see bp_covered_lanes); 2: the distance test
+// uses cover bitmaps.
+template <int MODE>
 __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, WarpRegion &wr,
                                 unsigned long long &bytes)
 {
@@ -948,7 +1015,7 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
         // t's row for a lane per candidate, in the bytes of the label stage
         ulonglong2 *lts = reinterpret_cast<ulonglong2 *>(wr.sh);
         uint32_t *ltd = wr.sh + MAX_BP * 4;
-        const bool lanes = LANES && iter <= BP_LANE_MAX_ITER && nsurv >= BP_LANE_MIN;
+        const bool lanes = MODE >= 1 && iter <= BP_LANE_MAX_ITER && nsurv >= BP_LANE_MIN;
         if (lanes) {
             lts[lane] = ts0;
             lts[lane + 32] = ts1;
@@ -1002,10 +1069,11 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
     uint32_t nadd = 0;
     if (nsurv) {
         uint32_t nst = 0;
+        const uint32_t room = SMALL_CAP - (MODE == 2 ? MAX_BATCH / 32 : 0u);
         // stage labels with d < iter from list position `from`; returns where it stopped
         auto stage = [&](uint32_t from) -> uint32_t {
             uint32_t cnt = 0, j = from;
-            while (j < len && cnt + 32 <= (uint32_t)SMALL_CAP) {
+            while (j < len && cnt + 32 <= room) {
                 // 4 chunks loaded before any is staged: one round trip for all
                 // (label loop of R-MAT s20, lists of 100 labels on average:
                 // 126.7 -> 122.8 ms)
@@ -1019,7 +1087,7 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    if (j >= len || cnt + 32 > (uint32_t)SMALL_CAP) break;
+                    if (j >= len || cnt + 32 > room) break;
                     const bool sm = dd[u] < iter;
                     const uint32_t m = __ballot_sync(FULL, sm);
                     if (sm) {
@@ -1036,7 +1104,72 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
             bytes += (uint64_t)min(j, len) - from + 4ull * cnt;
             return min(j, len);
         };
-        uint32_t next = stage(0);
+        if (MODE == 2) {
+            // all candidates at once: their batch bitmap (lane's 16 bytes of it,
+            // `open`) against the rows of the staged labels, 32 / G labels per
+            // load step and BM_LOADS steps in flight.  Exact up to slack
+            // BM_SLACKS; candidates left at a deeper level go on to the
+            // walk below.
+            uint32_t *open_w = wr.open();
+            const uint32_t G = d.words / 4, sub = lane & (G - 1), grp = lane / G, per = 32 / G;
+            for (uint32_t x = lane; x < d.words; x += 32) open_w[x] = 0;
+            __syncwarp();
+            for (uint32_t c = lane; c < nsurv; c += 32) atomicOr(&open_w[wr.offered[c] >> 5], 1u << (wr.offered[c] & 31));
+            __syncwarp();
+            uint4 open = *reinterpret_cast<const uint4 *>(open_w + sub * 4);
+            bool left = true;
+            for (uint32_t from = 0; from < len && left;) {
+                from = stage(from);
+                for (uint32_t k0 = 0; k0 < nst && left; k0 += per * BM_LOADS) {
+                    const bool any = open.x | open.y | open.z | open.w;
+                    uint4 v[BM_LOADS];
+#pragma unroll
+                    for (int u = 0; u < BM_LOADS; ++u) {
+                        const uint32_t k = k0 + u * per + grp;
+                        v[u] = make_uint4(0, 0, 0, 0);
+                        if (any && k < nst)
+                            v[u] = *reinterpret_cast<const uint4 *>(
+                                bc.bm + ((uint64_t)wr.sh[k] * BM_SLACKS + min((uint32_t)wr.sd[k], BM_SLACKS) - 1u) * d.words +
+                                sub * 4);
+                    }
+#pragma unroll
+                    for (int u = 0; u < BM_LOADS; ++u) {
+                        open.x &= ~v[u].x;
+                        open.y &= ~v[u].y;
+                        open.z &= ~v[u].z;
+                        open.w &= ~v[u].w;
+                    }
+                    // the lanes with the same 16 bytes agree
+                    for (uint32_t o = G; o < 32; o <<= 1) {
+                        open.x &= __shfl_xor_sync(FULL, open.x, o);
+                        open.y &= __shfl_xor_sync(FULL, open.y, o);
+                        open.z &= __shfl_xor_sync(FULL, open.z, o);
+                        open.w &= __shfl_xor_sync(FULL, open.w, o);
+                    }
+                    left = __any_sync(FULL, open.x | open.y | open.z | open.w);
+                }
+                __syncwarp();
+            }
+            if (grp == 0) *reinterpret_cast<uint4 *>(open_w + sub * 4) = open;
+            __syncwarp();
+            uint32_t k = 0;
+            for (uint32_t c0 = 0; c0 < nsurv; c0 += 32) {
+                const uint32_t c = c0 + lane;
+                const uint16_t idx = c < nsurv ? wr.offered[c] : (uint16_t)0;
+                const bool keep = c < nsurv && (open_w[idx >> 5] >> (idx & 31) & 1u);
+                const uint32_t km = __ballot_sync(FULL, keep);
+                __syncwarp();
+                if (keep) wr.offered[k + __popc(km & ((1u << lane) - 1u))] = idx;
+                k += __popc(km);
+                __syncwarp();
+            }
+            nsurv = k;
+            if (iter <= BM_SLACKS) {
+                nadd = k;
+                nsurv = 0;
+            }
+        }
+        uint32_t next = nsurv ? stage(0) : len;
         const bool whole = next >= len;
         bytes += 12;
         for (uint32_t c0 = 0; c0 < nsurv; c0 += 32) {
@@ -1130,6 +1263,7 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
             UD_AT(d.pool_hub, base + len + j, d.pool_cap, 2) = s + idx;
             UD_AT(d.pool_dist, base + len + j, d.pool_cap, 2) = (uint8_t)iter;
             if (is_root) UD_AT(bc.dm, (uint64_t)(t - s) * bc.dn + (s + idx - bc.base), (uint64_t)d.B * bc.dn, 4) = (uint8_t)iter;
+            if (MODE == 2 && is_root) bm_set(bc.bm, d.words, s + idx, t - s, iter);
             mn = min(mn, s + idx);
         }
         mn = warp_min_u32(mn);
@@ -1153,7 +1287,7 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
 
 // Pull phase of a level: heavy tails block-by-block, then light tails
 // warp-by-warp.  Ends with the block converged.
-template <bool LANES>
+template <int MODE>
 __device__ void pull_phase(const UnwDev &d, const PullArgs &a, unsigned char *pull_smem)
 {
     const int lane = threadIdx.x & 31;
@@ -1165,7 +1299,7 @@ __device__ void pull_phase(const UnwDev &d, const PullArgs &a, unsigned char *pu
         // that its scan and tests spread over 8 warps instead of one
         HeavyRegion hs = heavy_region(pull_smem, d.words, d.B);
         for (uint32_t q = blockIdx.x; q < hcnt + cnt; q += gridDim.x) {
-            pull_heavy_tail(d, a, q < hcnt ? a.htails[q] : a.tails[q - hcnt], hs, bytes);
+            pull_heavy_tail<MODE>(d, a, q < hcnt ? a.htails[q] : a.tails[q - hcnt], hs, bytes);
             __syncthreads();
         }
         if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_PULL], bytes);
@@ -1183,12 +1317,12 @@ __device__ void pull_phase(const UnwDev &d, const PullArgs &a, unsigned char *pu
                 const uint32_t q = hq;
                 __syncthreads();
                 if (q >= hcnt) break;
-                pull_heavy_tail(d, a, a.htails[q], hs, bytes);
+                pull_heavy_tail<MODE>(d, a, a.htails[q], hs, bytes);
                 __syncthreads();
             }
         } else {
             for (uint32_t q = blockIdx.x; q < hcnt; q += gridDim.x) {
-                pull_heavy_tail(d, a, a.htails[q], hs, bytes);
+                pull_heavy_tail<MODE>(d, a, a.htails[q], hs, bytes);
                 __syncthreads();
             }
         }
@@ -1196,11 +1330,11 @@ __device__ void pull_phase(const UnwDev &d, const PullArgs &a, unsigned char *pu
     }
     WarpRegion wr = warp_region(pull_smem, d.words, d.B, threadIdx.x >> 5);
     if (a.tail_q) {
-        for_claimed<0>(cnt, a.tail_q, [&](uint32_t q) { pull_light_tail<LANES>(d, a, a.tails[q], wr, bytes); });
+        for_claimed<0>(cnt, a.tail_q, [&](uint32_t q) { pull_light_tail<MODE>(d, a, a.tails[q], wr, bytes); });
     } else {
         const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
         for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < cnt; q += nw)
-            pull_light_tail<LANES>(d, a, a.tails[q], wr, bytes);
+            pull_light_tail<MODE>(d, a, a.tails[q], wr, bytes);
     }
     if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_PULL], bytes);
     __syncthreads();

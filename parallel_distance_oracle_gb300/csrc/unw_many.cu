@@ -172,7 +172,7 @@ __device__ void many_bookkeep(const UnwDev &d, ManyCtl *c, const ManyBufs &bf, u
     }
 }
 
-template <bool LANES>
+template <int MODE>
 __global__ void __launch_bounds__(PULL_THREADS, 4) many_loop_kernel(UnwDev d, ManyCtl *c, ManyBufs bf)
 {
     extern __shared__ __align__(16) unsigned char pull_smem[];
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) many_loop_kernel(UnwDev d, Ma
         } else {
             many_root_step(d, bf, c, bf.rr, vload(&c->rr_cnt), L);
         }
-        pull_phase<LANES>(d, a, pull_smem);
+        pull_phase<MODE>(d, a, pull_smem);
         if (leader) {
             c->tcnt[(L + 2) % 3] = 0;
             c->hcnt[(L + 2) % 3] = 0;
@@ -432,7 +432,7 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     PADO_CUDA(cudaEventRecord(e0, s));
     try {
         if (active) {
-            const void *kfn = hubs ? (const void *)many_loop_kernel<false> : (const void *)many_loop_kernel<true>;
+            const void *kfn = hubs ? (const void *)many_loop_kernel<0> : (const void *)many_loop_kernel<1>;
             PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             int dev = 0, sms = 0, per_sm = 0;
             PADO_CUDA(cudaGetDevice(&dev));
