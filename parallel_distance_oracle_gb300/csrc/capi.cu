@@ -290,7 +290,6 @@ void build_ingested(pado_index *h, pado::IngestResult &r, uint32_t K, uint32_t B
 
 constexpr uint64_t EXPORT_STAGE_BYTES = 32ull << 20;
 
-using pado::download_bytes;
 using pado::mapped_host;
 
 // Export in original-id order: vertex v takes the list (and BP row) of rank[v].
@@ -1071,11 +1070,12 @@ int pado_export(const pado_index *h, uint64_t *off, uint32_t *hub, void *dist, u
         cudaStream_t s = cudaStreamPerThread;
         if (!h->rank.n) {
             // ids are ranks: the store is already in export order
-            download_bytes(off, h->store.off.p, (uint64_t)(n + 1) * 8, s);
-            download_bytes(hub, h->store.hub.p, tot * 4, s);
-            download_bytes(dist, ddist, tot * dsz, s);
-            if (K && bp_dist) download_bytes(bp_dist, h->bpd.p, (uint64_t)n * K, s);
-            if (K && bp_sets) download_bytes(bp_sets, h->bps.p, (uint64_t)n * K * 16, s);
+            pado::download_all({{off, h->store.off.p, ((uint64_t)n + 1) * 8},
+                                {hub, h->store.hub.p, tot * 4},
+                                {dist, ddist, tot * dsz},
+                                {bp_dist, h->bpd.p, bp_dist ? (uint64_t)n * K : 0},
+                                {bp_sets, h->bps.p, bp_sets ? (uint64_t)n * K * 16 : 0}},
+                               s);
             PADO_CUDA(cudaStreamSynchronize(s));
             return;
         }
@@ -1090,9 +1090,9 @@ int pado_export(const pado_index *h, uint64_t *off, uint32_t *hub, void *dist, u
         const bool staged = bytes <= EXPORT_STAGE_BYTES;
         {
             pado::PBuf<uint64_t> noff((uint64_t)n + 1, s);
-            if (tot < (1ull << 32)) {
+            const bool scanned = tot < (1ull << 32);
+            if (scanned) {
                 pado::export_offsets(n, h->rank.p, h->store.off.p, noff.p, s);
-                download_bytes(off, noff.p, ((uint64_t)n + 1) * 8, s);
             } else {
                 std::vector<uint64_t> roff(n + 1);
                 std::vector<uint32_t> rk(n);
@@ -1125,10 +1125,12 @@ int pado_export(const pado_index *h, uint64_t *off, uint32_t *hub, void *dist, u
                                 n, K, bp ? 1 : 0, h->rank.p, h->store.off.p, noff.p, h->store.hub.p,
                                 static_cast<const uint8_t *>(ddist), (uint32_t)dsz, h->bpd.p, h->bps.p, ghub, gdist, gbpd,
                                 gbps));
-            if (!ohub) download_bytes(hub, ghub, tot * 4, s);
-            if (!odist) download_bytes(dist, gdist, tot * dsz, s);
-            if (K && bp_dist && !obpd) download_bytes(bp_dist, gbpd, (uint64_t)n * K, s);
-            if (K && bp_sets && !obps) download_bytes(bp_sets, gbps, (uint64_t)n * K * 16, s);
+            pado::download_all({{off, noff.p, scanned ? ((uint64_t)n + 1) * 8 : 0},
+                                {hub, ghub, ohub ? 0 : tot * 4},
+                                {dist, gdist, odist ? 0 : tot * dsz},
+                                {bp_dist, gbpd, bp_dist && !obpd ? (uint64_t)n * K : 0},
+                                {bp_sets, gbps, bp_sets && !obps ? (uint64_t)n * K * 16 : 0}},
+                               s);
             PADO_CUDA(cudaStreamSynchronize(s));
         }
         pado::release_scratch(std::max(scratch_keep(), QUERY_POOL_KEEP));

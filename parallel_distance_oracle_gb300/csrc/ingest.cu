@@ -1084,8 +1084,55 @@ void release_scratch(uint64_t keep_bytes)
     PADO_CUDA(cudaMemPoolTrimTo(scratch_pool(), keep_bytes));
 }
 
-// Vertex v's share of an export in original-id order: the length of the list of
-// its rank; entry n closes the scan.
+// Offsets of an export in original-id order: vertex v has the list of rank[v].
+// One block, 4,096 vertices a step, four in a row per thread: a step is a gather
+// (rank, two offsets) and a block scan, all latency.
+__global__ void __launch_bounds__(1024) export_scan_kernel(const uint32_t *rank, const uint64_t *roff, uint32_t n,
+                                                           uint64_t *noff)
+{
+    __shared__ uint64_t wsum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t carry = 0;
+    for (uint64_t at = 0; at < n; at += 4096) {
+        const uint64_t v = at + 4ull * threadIdx.x;
+        uint64_t len[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t r = v + j < n ? rank[v + j] : 0u;
+            len[j] = v + j < n ? roff[r + 1] - roff[r] : 0ull;
+        }
+        const uint64_t own = len[0] + len[1] + len[2] + len[3];
+        uint64_t x = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        uint64_t before = 0, all = 0;
+        {
+            uint64_t z = wsum[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t y = __shfl_up_sync(0xffffffffu, z, o);
+                if (lane >= o) z += y;
+            }
+            all = __shfl_sync(0xffffffffu, z, 31);
+            before = __shfl_sync(0xffffffffu, z, (warp + 31) & 31);
+            if (warp == 0) before = 0;
+        }
+        uint64_t o = carry + before + x - own;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (v + j < n) noff[v + j] = o;
+            o += len[j];
+        }
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) noff[n] = carry;
+}
+
+// Larger exports: entry v of the scan's input; entry n closes it.
 __global__ void __launch_bounds__(256) export_len_kernel(const uint32_t *rank, const uint64_t *roff, uint32_t n,
                                                          uint32_t *len)
 {
@@ -1093,8 +1140,16 @@ __global__ void __launch_bounds__(256) export_len_kernel(const uint32_t *rank, c
         len[v] = v < n ? (uint32_t)(roff[rank[v] + 1] - roff[rank[v]]) : 0u;
 }
 
+// Up to here one block's scan (5 us and 5.5 more per 4,096 vertices) is faster than the
+// five launches of the other way (25 us).
+constexpr uint32_t EXPORT_SCAN_MAX = 16384;
+
 void export_offsets(uint32_t n, const uint32_t *rank, const uint64_t *roff, uint64_t *noff, cudaStream_t s)
 {
+    if (n <= EXPORT_SCAN_MAX) {
+        PADO_LAUNCH("export_scan_kernel", s, export_scan_kernel<<<1, 1024, 0, s>>>(rank, roff, n, noff));
+        return;
+    }
     PBuf<uint32_t> len((uint64_t)n + 1, s), sums(scan_sums_needed((uint64_t)n + 1), s);
     PADO_LAUNCH("export_len_kernel", s,
                 export_len_kernel<<<grid_for((uint64_t)n + 1, 256), 256, 0, s>>>(rank, roff, n, len.p));

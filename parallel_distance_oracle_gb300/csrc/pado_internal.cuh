@@ -223,7 +223,12 @@ EdgeTextParser read_edge_file(const char *path, bool weighted, cudaStream_t s);
 // pointer), and copies between host and device memory that the SMs carry out
 // when the host side is page-locked (the copy engines otherwise), enqueued on s.
 void *mapped_host(const void *p);
-void download_bytes(void *h, const void *d, uint64_t bytes, cudaStream_t s);
+struct HostCopy {
+    void *h;
+    const void *d;
+    uint64_t bytes;
+};
+void download_all(std::initializer_list<HostCopy> copies, cudaStream_t s);
 void upload_bytes(void *d, const void *h, uint64_t bytes, cudaStream_t s);
 
 // capi.cu: the calling thread's last-error message, and read-only access to
