@@ -67,7 +67,11 @@ namespace pado {
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int WPULL_WARPS = 4;
+// Warps of a pull block.  The loop takes blocks of eight where that leaves as many warps
+// resident as blocks of four do (shared memory decides: B up to 700 or so, and B = 2048):
+// half the blocks make the barriers cheaper (wrmat18, B = 512: a build 57.7 -> 55.2 ms).
+// At B = 1000 sixteen warps per SM fit instead of twenty: 68.3 ms against 61.8.
+constexpr int WPULL_WARPS = 4, WLOOP_WARPS = 8;
 constexpr int32_t RMIN_EMPTY = INT_MAX;
 // Tails of at least this degree are worked on by the whole grid: their heads
 // in items of WITEM adjacency entries, then a block each (see WTails).
@@ -474,7 +478,7 @@ __device__ __forceinline__ int32_t w_check_group(const WDev &d, uint32_t t, bool
 
 // The pull of one round (send_messages, pado_weighted_unv_unp.h:409-870, as
 // a pull).  Per-warp dynamic shared memory: rmin[B] int32, res[B] int32,
-// touched[B] u16.  Run by blocks of WPULL_WARPS warps.
+// touched[B] u16.
 // tq: the round's work counter for dynamic tail claiming (null: static
 // grid-stride assignment).  FIRST: batch 0, whose rounds are few, large and
 // need check (2) and the walk of long logs; the other batches' many small rounds
@@ -490,8 +494,9 @@ __device__ void w_pull_phase(const WDev &d, const uint32_t *tails, uint32_t cnt,
     const int w = threadIdx.x >> 5;
     const uint32_t B = d.B;
     int32_t *rmin = reinterpret_cast<int32_t *>(wsm) + (size_t)w * B;
-    int32_t *res = reinterpret_cast<int32_t *>(wsm) + (size_t)WPULL_WARPS * B + (size_t)w * B;
-    uint16_t *touched = reinterpret_cast<uint16_t *>(reinterpret_cast<int32_t *>(wsm) + (size_t)2 * WPULL_WARPS * B) +
+    const uint32_t bw = blockDim.x >> 5;
+    int32_t *res = reinterpret_cast<int32_t *>(wsm) + (size_t)bw * B + (size_t)w * B;
+    uint16_t *touched = reinterpret_cast<uint16_t *>(reinterpret_cast<int32_t *>(wsm) + (size_t)2 * bw * B) +
                         (size_t)w * B;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     const int cp = lid_cur & 1;
@@ -611,7 +616,7 @@ __device__ __noinline__ void w_heavy_items_phase(const WDev &d, const WTails &tl
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t B = d.B;
     int32_t *rmin = reinterpret_cast<int32_t *>(wsm) + (size_t)w * B;
-    uint16_t *touched = reinterpret_cast<uint16_t *>(reinterpret_cast<int32_t *>(wsm) + (size_t)2 * WPULL_WARPS * B) +
+    uint16_t *touched = reinterpret_cast<uint16_t *>(reinterpret_cast<int32_t *>(wsm) + (size_t)2 * (blockDim.x >> 5) * B) +
                         (size_t)w * B;
     for (uint32_t c = lane; c < B; c += 32) rmin[c] = RMIN_EMPTY;
     __syncwarp();
@@ -644,13 +649,14 @@ __device__ __noinline__ void w_heavy_finish_phase(const WDev &d, const uint32_t 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, cp = lid_cur & 1;
     const uint32_t B = d.B, below = (1u << lane) - 1u;
     int32_t *rmin = reinterpret_cast<int32_t *>(wsm);
-    int32_t *res = rmin + (size_t)WPULL_WARPS * B;
-    uint16_t *touched = reinterpret_cast<uint16_t *>(rmin + (size_t)2 * WPULL_WARPS * B);
+    const uint32_t bw = blockDim.x >> 5;
+    int32_t *res = rmin + (size_t)bw * B;
+    uint16_t *touched = reinterpret_cast<uint16_t *>(rmin + (size_t)2 * bw * B);
     for (uint32_t q = blockIdx.x; q < nheavy; q += gridDim.x) {
         const uint32_t t = heavy[q];
         int32_t *row = hmin + (uint64_t)q * B;
         __syncthreads();  // the previous tail's shared state is done with
-        for (uint32_t c = threadIdx.x; c < B; c += WPULL_WARPS * 32) {
+        for (uint32_t c = threadIdx.x; c < B; c += blockDim.x) {
             const int32_t x = __ldcg(row + c);
             rmin[c] = x == HMIN_EMPTY ? RMIN_EMPTY : x;
             if (x != HMIN_EMPTY) row[c] = HMIN_EMPTY;
@@ -672,7 +678,7 @@ __device__ __noinline__ void w_heavy_finish_phase(const WDev &d, const uint32_t 
         const uint32_t ntouch = sum[0], ng = (ntouch + 31) / 32;
         const uint64_t cbase = d.lab_off[t];
         const uint32_t clen = d.lab_len[t], vql = d.vq_len[t];
-        for (uint32_t g = w; g < ng; g += WPULL_WARPS) {
+        for (uint32_t g = w; g < ng; g += bw) {
             const uint32_t i = g * 32 + lane;
             const uint32_t c = i < ntouch ? touched[i] : 0u;
             const int32_t r = w_check_group<FIRST>(d, t, i < ntouch, c, rmin, s, b, cbase, clen, vql);
@@ -705,7 +711,7 @@ __device__ __noinline__ void w_heavy_finish_phase(const WDev &d, const uint32_t 
         __syncthreads();
         if (!sum[4]) continue;  // uniform; nothing committed
         const unsigned long long lpos = slpos;
-        for (uint32_t g = w; g < ng; g += WPULL_WARPS) {
+        for (uint32_t g = w; g < ng; g += bw) {
             // accepted and new roots of the groups before g
             uint32_t accb = 0, newb = 0;
             for (uint32_t j = lane; j < g; j += 32) {
@@ -739,7 +745,7 @@ __device__ __noinline__ void w_heavy_finish_phase(const WDev &d, const uint32_t 
                 d.act_stamp[cp][t] = lid_cur;
             }
         }
-        if (nacc) w_mark_head(d, t, mnacc, lid_cur + 1, next, w, WPULL_WARPS);
+        if (nacc) w_mark_head(d, t, mnacc, lid_cur + 1, next, w, bw);
     }
 }
 
@@ -1028,7 +1034,7 @@ struct WLoopBufs {
 // The heavy phases are functions of their own (the parameters in constant
 // memory can be passed by reference): inlined, their registers made the many
 // small rounds spill (55.5 ms against 54.1 ms on wrmat18).
-__global__ void __launch_bounds__(WPULL_WARPS * 32, 8) w_loop_kernel(const __grid_constant__ WDev d, WLoopCtl *c, const __grid_constant__ WLoopBufs bf)
+__global__ void __launch_bounds__(WLOOP_WARPS * 32, 4) w_loop_kernel(const __grid_constant__ WDev d, WLoopCtl *c, const __grid_constant__ WLoopBufs bf)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
     const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
@@ -1323,20 +1329,25 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
             WLoopBufs bf{{tails.p, tails2.p, tails3.p}, {ht[0].p, ht[1].p, ht[2].p}, {news.p, news2.p},
                          {hi[0].p, hi[1].p, hi[2].p}, hmin.p, rr.p, retry.p, heavy.p, nbatches};
             const void *kfn = (const void *)w_loop_kernel;
-            PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pull_smem));
-            int dev = 0, sms = 0, per_sm = 0;
+            const size_t loop_smem = pull_smem * WLOOP_WARPS / WPULL_WARPS;
+            PADO_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)loop_smem));
+            int dev = 0, sms = 0, per_sm = 0, wide = 0;
             PADO_CUDA(cudaGetDevice(&dev));
             PADO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             PADO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, WPULL_WARPS * 32, pull_smem));
-            PADO_CHECK(per_sm >= 1, PADO_E_CUDA, "weighted labeling loop kernel cannot be resident");
-            const unsigned grid = (unsigned)(sms * std::min(per_sm, 8));
+            PADO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide, kfn, WLOOP_WARPS * 32, loop_smem));
+            PADO_CHECK(per_sm >= 1 || wide >= 1, PADO_E_CUDA, "weighted labeling loop kernel cannot be resident");
+            const bool big = wide * WLOOP_WARPS >= per_sm * WPULL_WARPS;
+            const int threads = 32 * (big ? WLOOP_WARPS : WPULL_WARPS);
+            const unsigned grid = (unsigned)(sms * (big ? wide : per_sm));
             WLoopCtl h{};
             WLoopCtl *cptr = ctl.p;
             for (int launch = 0;; ++launch) {
                 PADO_CHECK(launch < 512, PADO_E_NOMEM, "round log or label pool could not be grown enough");
                 void *args[] = {&d, &cptr, &bf};
                 PADO_LAUNCH("w_loop_kernel", s,
-                            PADO_CUDA(cudaLaunchCooperativeKernel(kfn, grid, WPULL_WARPS * 32, args, pull_smem, s)));
+                            PADO_CUDA(cudaLaunchCooperativeKernel(kfn, grid, threads, args,
+                                                                  big ? loop_smem : pull_smem, s)));
                 PADO_CUDA(cudaMemcpyAsync(&h, ctl.p, sizeof(WLoopCtl), cudaMemcpyDeviceToHost, s));
                 PADO_CUDA(cudaStreamSynchronize(s));
                 if (h.status & ST_BARRIER_TIMEOUT)
