@@ -30,7 +30,7 @@
 //       child step); slots so reached get level d+1 and put w on level d+1.
 // The child step pulls along the same edges the reference pushes along, and
 // every update is an OR, so the rows are bit-identical.  Vertices of degree
-// >= HEAVY are worked on by a whole block (8 warps over the neighbours, one
+// >= st.heavy are worked on by a whole block (8 warps over the neighbours, one
 // shared-memory reduction).  For many graphs in one union id space, slot i
 // holds every graph's i-th root: the graphs are disjoint, so their BFSes
 // never meet.
@@ -44,10 +44,23 @@ namespace pado {
 namespace {
 
 constexpr unsigned FULL_MASK = 0xffffffffu;
-constexpr uint32_t HEAVY = 2048;     // vertices worked on by a whole block
 constexpr int BP_THREADS = 256;
 constexpr int BP_WARPS = BP_THREADS / 32;
 constexpr int NB = 4;                // neighbours whose rows are loaded together
+
+// The degree from which a vertex is worked on by a whole block: as low as leaves about one
+// such vertex per block of the grid.  In a small graph a hub's neighbours, 32 at a time, are
+// a warp's chain that every level waits for; in a large one blocks for mid-degree
+// vertices would queue behind each other.  Judged by the degrees at doubling ids past the
+// grid (ids are ranks, most often by degree).  Against 2,048 for all (R-MAT, us of the
+// loop): s10/ef8 195 -> 137, s12/ef8 368 -> 174, s14/ef16 766 -> 358, s16/ef8 901 -> 608,
+// s18 and up the same.
+uint32_t heavy_degree(const HostGraph &hg, uint32_t grid)
+{
+    uint32_t t = 64;
+    for (uint64_t v = grid; v < hg.n; v *= 2) t = std::max(t, (uint32_t)(hg.off[v + 1] - hg.off[v]));
+    return std::min(t, 2048u);
+}
 
 // Slots where a vertex is on level `lvl`; valid only if `lvl` matches the level
 // being read (the two parity buffers are never cleared).
@@ -58,6 +71,7 @@ struct LevelMask {
 
 struct MsState {
     uint32_t n, K;
+    uint32_t heavy;        // vertices of at least this degree are worked on by a whole block
     const uint32_t *off;
     const uint32_t *adj;
     uint8_t *bpd;          // [n][K]: level per slot, 255 = unreached (final rows)
@@ -83,7 +97,7 @@ __device__ __forceinline__ unsigned long long level_bits(const MsState &st, uint
 
 __device__ __forceinline__ void vlist_append(const MsState &st, const VList &l, uint32_t v)
 {
-    const bool heavy = st.off[v + 1] - st.off[v] >= HEAVY;
+    const bool heavy = st.off[v + 1] - st.off[v] >= st.heavy;
     if (heavy)
         l.heavy[agg_append_by(&l.cnt[1], 1u)] = v;
     else
@@ -441,7 +455,13 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
         // empty masks stamped with a level no BFS reaches
         PADO_LAUNCH("bp_init_kernel", s, bp_init_kernel<<<grid_for(n, 256), 256, 0, s>>>(lm0.p, lm1.p, n));
         fstamp.fill_bytes(0xff, s);
-        MsState st{n, K, g.off.p, g.adj.p, d_bpd, reinterpret_cast<ulonglong2 *>(d_bps), reach.p,
+        int dev = 0, sms = 0, per_sm = 0;
+        PADO_CUDA(cudaGetDevice(&dev));
+        PADO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        PADO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_loop_kernel, BP_THREADS, 0));
+        PADO_CHECK(per_sm >= 1, PADO_E_CUDA, "bit-parallel loop kernel cannot be resident");
+        const unsigned grid = (unsigned)(sms * per_sm);
+        MsState st{n, K, heavy_degree(hg, grid), g.off.p, g.adj.p, d_bpd, reinterpret_cast<ulonglong2 *>(d_bps), reach.p,
                    {lm0.p, lm1.p}, cstamp.p, fstamp.p, work_counters()};
 
         // seeds and the frontiers of levels 0 (roots) and 1 (selected neighbours), deduplicated
@@ -455,7 +475,7 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
                 sv.push_back(x.v);
                 sl.push_back(x.lvl);
                 sb.push_back(x.bits);
-                const bool heavy = hg.off[x.v + 1] - hg.off[x.v] >= HEAVY;
+                const bool heavy = hg.off[x.v + 1] - hg.off[x.v] >= st.heavy;
                 if (x.lvl == 0 && !in0[x.v]) {
                     in0[x.v] = 1;
                     f0[heavy].push_back(x.v);
@@ -498,17 +518,11 @@ BpResult bp_run(const HostGraph &hg, const DevGraph &g, uint32_t K, const std::v
         h.front[1][0] = (uint32_t)f1[0].size();
         h.front[1][1] = (uint32_t)f1[1].size();
         ctl.upload(&h, 1, s);
-        int dev = 0, sms = 0, per_sm = 0;
-        PADO_CUDA(cudaGetDevice(&dev));
-        PADO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        PADO_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_loop_kernel, BP_THREADS, 0));
-        PADO_CHECK(per_sm >= 1, PADO_E_CUDA, "bit-parallel loop kernel cannot be resident");
         BpCtl *cp = ctl.p;
         BpLists lists{{fl[0].p, fl[1].p, fl[2].p}, {fh[0].p, fh[1].p, fh[2].p}, cl.p, ch.p};
         void *args[] = {&st, &cp, &lists};
         PADO_LAUNCH("bp_loop_kernel", s,
-                    PADO_CUDA(cudaLaunchCooperativeKernel((const void *)bp_loop_kernel, sms * per_sm, BP_THREADS, args, 0,
-                                                          s)));
+                    PADO_CUDA(cudaLaunchCooperativeKernel((const void *)bp_loop_kernel, grid, BP_THREADS, args, 0, s)));
         PADO_CUDA(cudaMemcpyAsync(&h, ctl.p, sizeof(h), cudaMemcpyDeviceToHost, s));
         PADO_LAUNCH("bp_finish_kernel", s,
                     bp_finish_kernel<<<grid_for((uint64_t)n * K, 256), 256, 0, s>>>(st));
