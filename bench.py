@@ -749,12 +749,13 @@ def ingest_cpu(scale: int):
 
 
 # Algorithmic bytes of one launch of the ingest kernels, L = directed entries
-# (2 per edge), m = edges: the keys each radix pass reads and writes, the
-# keys' build from the edge list and the adjacency read out of them.
+# (2 per edge), m = edges: the keys' build from the edge list and the keys each
+# radix pass reads and writes; the last of the entries' five passes writes the
+# adjacency (4 bytes) instead of keys.
 def ingest_kernel_bytes(kernel: str, m: int):
     L = 2 * m
-    return {"rs_scatter_kernel": 16 * L, "rs_hist_kernel": 8 * L, "entry_key_kernel": 8 * m + 8 * m + 8 * L,
-            "extract_kernel": 12 * L, "degree_kernel": 8 * m + 16 * m}.get(kernel)
+    return {"rs_scatter_kernel": (4 * 16 + 12) * L // 5, "rs_hist_kernel": 8 * L,
+            "entry_key_kernel": 8 * m + 8 * m + 8 * L, "degree_kernel": 8 * m + 16 * m}.get(kernel)
 
 
 def run_ingest(args):
