@@ -1,5 +1,6 @@
-"""Calls that the library refuses with a status, without reading outside their
-arrays; the device labels as before afterwards."""
+"""Calls with arguments that are not what the library asks for: refused with a
+status, or answered, without an access outside their arrays; the library works as
+before afterwards."""
 from __future__ import annotations
 
 import ctypes as C
@@ -48,3 +49,28 @@ def test_malformed_csr(cuda_ok, weighted, off, first):
     rank = G.degree_rank(g)
     got, ref = pado.WeightedVertexCentricPLL(g, rank, batch=64).export(), orc.w_label(g, rank, 64)
     assert np.array_equal(got.off, ref.off) and np.array_equal(got.hub, ref.hub)
+
+
+@pytest.mark.parametrize("k", [1, 300, 20000])
+@pytest.mark.parametrize("which", ["a", "b", "out"])
+def test_query_with_a_device_array(cuda_ok, which, k):
+    """pado_query takes host arrays.  A device array in the place of one goes
+    through the runtime's copies: a status or the right distances, and the host
+    never touches it."""
+    import torch
+
+    from parallel_distance_oracle_gb300 import _lib as L
+    from parallel_distance_oracle_gb300 import pado
+    g = G.rmat(9, 6, 12)
+    idx = pado.VertexCentricPLL(g, G.degree_rank(g), bp_roots=8, batch=64)
+    rng = np.random.Generator(np.random.PCG64(k))
+    a, b = (rng.integers(0, g.n, k).astype(np.uint32) for _ in range(2))
+    ref, out = idx.query(a, b), np.zeros(k, np.uint8)
+    host = {"a": a.view(np.int32), "b": b.view(np.int32), "out": out}
+    dev = torch.from_numpy(host[which]).cuda()
+    torch.cuda.synchronize()
+    p = {x: L.ptr(y) for x, y in host.items()} | {which: C.c_void_p(dev.data_ptr())}
+    st = L.lib.pado_query(idx._need(), k, p["a"], p["b"], p["out"])
+    assert st != 0 or np.array_equal(dev.cpu().numpy() if which == "out" else out, ref)
+    # the caller's own arrays are untouched and ordinary calls go on
+    assert np.array_equal(idx.query(a, b), ref)
