@@ -317,14 +317,19 @@ inline uint64_t debug_pool_entries()
 // The label pool starts at 256 entries per vertex (1.3 KB/vertex unweighted,
 // capped at 2^31 entries): enough for a social-graph labeling plus its list
 // relocations in one persistent launch, so growth relaunches are rare.  Graphs
-// without hubs (has_hubs) carry about n / 30 labels per vertex (661 at n =
+// without hubs (has_hubs) may carry about n / 30 labels per vertex (661 at n =
 // 20,011, 1,749 at 50,000), twice that and more with relocations: n / 8 entries
-// per vertex, at most 4,096, spare them the three growths 256 cost (0.4 ms each).
+// per vertex spare them the growths that 256 cost (0.4 ms each).  Such a graph may
+// as well be a tree with a dozen labels per vertex, so this stops at 512 MiB
+// (n = 29,308, where 256 per vertex are 36 MiB; from n = 419,431 on 256 are more).
+constexpr uint64_t NO_HUBS_POOL_ENTRIES = (512ull << 20) / 5;
 inline uint64_t initial_pool_entries(uint32_t n, bool hubs = true)
 {
     const uint64_t dbg = debug_pool_entries();
-    const uint64_t per = hubs ? 256 : std::min<uint64_t>(std::max<uint64_t>(n / 8, 256), 4096);
-    return dbg ? dbg : std::min<uint64_t>(std::max<uint64_t>(n * per, 1u << 22), 1ull << 31);
+    if (dbg) return dbg;
+    uint64_t e = std::max<uint64_t>((uint64_t)n * 256, 1u << 22);
+    if (!hubs) e = std::max(e, std::min((uint64_t)n * n / 8, NO_HUBS_POOL_ENTRIES));
+    return std::min<uint64_t>(e, 1ull << 31);
 }
 // The weighted round logs start at 128 entries per vertex (1 KB per vertex
 // for both parities): the busiest rounds of the first batch of a social graph

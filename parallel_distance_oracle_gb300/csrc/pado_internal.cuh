@@ -96,15 +96,16 @@ struct LabelRun {
 // Vertices of ids [lo, hi) that have hubs among them, judged by the first one
 // (the largest degree in a degree order): more than 8 times their average
 // degree.  R-MAT graphs lie above (16 times at 1,024 vertices, 2,000 at s20),
-// random graphs and grids with shortcuts below (3 and 2 times).  It only picks
-// the variant of the label loop that is faster on such graphs.
+// random graphs and grids with shortcuts below (3 and 2 times).  It picks the
+// variant of the label loop that is faster on such graphs and the label pool that
+// it starts with (initial_pool_entries).
 inline bool has_hubs(const HostGraph &hg, uint32_t lo, uint32_t hi)
 {
     return hi > lo && (uint64_t)(hg.off[lo + 1] - hg.off[lo]) * (hi - lo) > 8ull * (hg.off[hi] - hg.off[lo]);
 }
 
 // unw.cu: batched pruned BFS labeling (pado_unw_unv_unp.h:425-1118); hubs: see
-// has_hubs.
+// has_hubs.  Where the variant without hubs cannot have its memory, the other is run.
 LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<uint8_t> &used,
                    const uint8_t *d_bpd, const uint64_t *d_bps, bool hubs, LabelStore &out, cudaStream_t s);
 

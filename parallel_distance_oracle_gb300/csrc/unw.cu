@@ -309,10 +309,8 @@ __global__ void __launch_bounds__(256) finalize_kernel(UnwDev d, const uint64_t 
     finalize_phase(d, fin_off, fin_hub, fin_dist, nullptr, nullptr);
 }
 
-}  // namespace
-
-LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<uint8_t> &used,
-                   const uint8_t *d_bpd, const uint64_t *d_bps, bool hubs, LabelStore &out, cudaStream_t s)
+LabelRun label_graph(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<uint8_t> &used,
+                     const uint8_t *d_bpd, const uint64_t *d_bps, bool hubs, LabelStore &out, cudaStream_t s)
 {
     LabelRun run;
     const uint32_t n = g.n;
@@ -721,6 +719,24 @@ LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<
     cudaEventDestroy(e1);
     release_phase.emplace("label release");
     return run;
+}
+
+}  // namespace
+
+LabelRun unw_label(const DevGraph &g, uint32_t K, uint32_t B, const std::vector<uint8_t> &used,
+                   const uint8_t *d_bpd, const uint64_t *d_bps, bool hubs, LabelStore &out, cudaStream_t s)
+{
+    if (!hubs) {
+        try {
+            return label_graph(g, K, B, used, d_bpd, d_bps, false, out, s);
+        } catch (const Error &e) {
+            if (e.code != PADO_E_NOMEM) throw;
+        }
+        // its pool, bitmaps and padded rows did not fit: again without them
+        cudaGetLastError();
+        out = LabelStore();
+    }
+    return label_graph(g, K, B, used, d_bpd, d_bps, true, out, s);
 }
 
 }  // namespace pado
