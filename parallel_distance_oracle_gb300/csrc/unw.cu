@@ -357,12 +357,15 @@ LabelRun label_graph(const DevGraph &g, uint32_t K, uint32_t B, const std::vecto
     zeros.add(counters, 8);
     zeros.add(status, 1);
     zeros.add(ctl, 1);
-    DBuf<uint8_t> d_used, bpmin, bpdp;  // bpdp: only when rows of K bytes are not whole 16
+    // padded BP rows: only for the instances that read them, and when rows of K bytes
+    // are not whole 16
+    const bool padded = !hubs && !host_loop && K % 16;
+    DBuf<uint8_t> d_used, bpmin, bpdp;
     DBuf<uint32_t> last_min0, last_min1, ind, front0, front1, tails, htails, tails2, htails3, retry, roots, rr, d_broots,
         d_boff;
     ws.add(d_used, std::max<uint32_t>(n, 1));
     ws.add(bpmin, std::max<uint32_t>(n, 1));
-    ws.add(bpdp, K % 16 ? (uint64_t)n * ((K + 15) / 16 * 16) : 1);
+    ws.add(bpdp, padded ? (uint64_t)n * ((K + 15) / 16 * 16) : 1);
     ws.add(last_min0, n);
     ws.add(last_min1, n);
     ws.add(ind, (uint64_t)n * words);
@@ -406,10 +409,10 @@ LabelRun label_graph(const DevGraph &g, uint32_t K, uint32_t B, const std::vecto
     d.bpd = d_bpd;
     d.bps = d_bps;
     d.kp = (K + 15) / 16 * 16;
-    d.bpdp = d.kp == K ? d_bpd : bpdp.p;
+    d.bpdp = padded ? bpdp.p : d_bpd;
     if (K && n)
         PADO_LAUNCH("bpmin_kernel", s,
-                    bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p, d.kp == K ? nullptr : bpdp.p,
+                    bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p, padded ? bpdp.p : nullptr,
                                                                   d.kp));
     d.bpmin = bpmin.p;
     d.pool_hub = pool_hub.p;

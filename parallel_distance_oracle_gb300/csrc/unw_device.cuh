@@ -58,7 +58,8 @@ struct UnwDev {
     const uint8_t *bpd;
     const uint64_t *bps;
     const uint8_t *bpmin;   // per vertex: least BP distance over the roots (255: none)
-    const uint8_t *bpdp;    // [n][kp]: bpd with rows of whole 16 bytes, 255 past K (bpd itself when K is such)
+    const uint8_t *bpdp;    // [n][kp]: bpd with rows of whole 16 bytes, 255 past K (bpd itself when K is such);
+                            // read by MODE 1 and up only
     uint32_t kp;
     uint32_t *pool_hub;
     uint8_t *pool_dist;

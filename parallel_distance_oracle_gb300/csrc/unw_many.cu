@@ -326,7 +326,10 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     zeros.add(last1, n);
     for (DBuf<uint32_t> *x : {&lab_len, &lab_cap, &tail_stamp, &ind_stamp}) zeros.add(*x, n);
     zeros.add(status, 1);
-    DBuf<uint8_t> d_used, bpmin, bpdp;  // bpdp: only when rows of K bytes are not whole 16
+    // padded BP rows: only for the instance that reads them, and when rows of K bytes are
+    // not whole 16
+    const bool padded = !hubs && K % 16;
+    DBuf<uint8_t> d_used, bpmin, bpdp;
     DBuf<uint32_t> last_min0, last_min1, ind, tl0, tl1, tl2, th0, th1, th2, rretry, tretry, rq0b, rq1b, zq0b, zq1b, rr;
     DBuf<uint32_t> d_broots, d_bcnt, d_gbase;
     DBuf<GDesc> d_gd;
@@ -334,7 +337,7 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     DBuf<ManyCtl> ctl;
     ws.add(d_used, std::max<uint32_t>(n, 1));
     ws.add(bpmin, std::max<uint32_t>(n, 1));
-    ws.add(bpdp, K % 16 ? (uint64_t)n * ((K + 15) / 16 * 16) : 1);
+    ws.add(bpdp, padded ? (uint64_t)n * ((K + 15) / 16 * 16) : 1);
     ws.add(ind, (uint64_t)n * words);
     for (DBuf<uint32_t> *x : {&last_min0, &last_min1, &tl0, &tl1, &tl2, &th0, &th1, &th2, &rretry, &tretry, &rq0b, &rq1b,
                               &zq0b, &zq1b, &rr})
@@ -382,10 +385,10 @@ LabelRun unw_label_many(const DevGraph &g, const std::vector<uint32_t> &gbase, u
     d.bpd = d_bpd;
     d.bps = d_bps;
     d.kp = (K + 15) / 16 * 16;
-    d.bpdp = d.kp == K ? d_bpd : bpdp.p;
+    d.bpdp = padded ? bpdp.p : d_bpd;
     if (K && n)
         PADO_LAUNCH("bpmin_kernel", s,
-                    bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p, d.kp == K ? nullptr : bpdp.p,
+                    bpmin_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_bpd, n, K, bpmin.p, padded ? bpdp.p : nullptr,
                                                                   d.kp));
     d.bpmin = bpmin.p;
     d.pool_hub = pool_hub.p;

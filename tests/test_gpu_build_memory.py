@@ -1,6 +1,7 @@
-"""The label pool that a build starts with on graphs without hubs: larger than
-with hubs, but bounded, and a build that cannot have it (or what else its
-variant of the loop allocates) goes on with what a graph with hubs gets."""
+"""Device memory of a build.  The label pool that it starts with on graphs without
+hubs: larger than with hubs, but bounded, and a build that cannot have it (or what
+else its variant of the loop allocates) goes on with what a graph with hubs gets.
+Tables that only one variant reads are that variant's."""
 from __future__ import annotations
 
 import ctypes as C
@@ -19,15 +20,11 @@ pytestmark = pytest.mark.gpu
 E_NOMEM = 2
 
 
-def test_memory_of_a_tree(cuda_ok):
-    """A binary tree of 524,287 vertices has a dozen labels per vertex; a build that
-    starts with 256 pool entries per vertex holds 2.4 GB."""
+def _peak(build):
+    """Device bytes held at most during build(), run three times after a first one
+    (which loads the library's kernels)."""
     import torch
-
-    from parallel_distance_oracle_gb300 import pado
-    n = (1 << 19) - 1
-    v = np.arange(1, n)
-    g = G.csr_from_edges(n, (v - 1) // 2, v)
+    build()
     torch.cuda.synchronize()
     free0 = least = torch.cuda.mem_get_info()[0]
     done = threading.Event()
@@ -42,11 +39,33 @@ def test_memory_of_a_tree(cuda_ok):
     t.start()
     try:
         for _ in range(3):
-            pado.VertexCentricPLL(g, np.arange(n, dtype=np.uint32), bp_roots=64, batch=1024).close()
+            build()
     finally:
         done.set()
         t.join()
-    assert free0 - least < 4e9
+    return free0 - least
+
+
+def test_memory_of_a_tree(cuda_ok):
+    """A binary tree of 524,287 vertices has a dozen labels per vertex; a build that
+    starts with 256 pool entries per vertex holds 2.4 GB."""
+    from parallel_distance_oracle_gb300 import pado
+    n = (1 << 19) - 1
+    v = np.arange(1, n)
+    g = G.csr_from_edges(n, (v - 1) // 2, v)
+    rank = np.arange(n, dtype=np.uint32)
+    assert _peak(lambda: pado.VertexCentricPLL(g, rank, bp_roots=64, batch=1024).close()) < 4e9
+
+
+def test_memory_of_padded_rows(cuda_ok):
+    """With hubs nothing reads the 16-byte rows of BP distances: K = 50 holds two
+    roots' rows (34 bytes a vertex) more than K = 48, not 64 bytes on top."""
+    from parallel_distance_oracle_gb300 import pado
+    n = 1 << 21
+    g = G.csr_from_edges(n, np.zeros(n - 1, np.int64), np.arange(1, n))
+    rank = np.arange(n, dtype=np.uint32)
+    peak = [_peak(lambda: pado.VertexCentricPLL(g, rank, bp_roots=K, batch=1024).close()) for K in (48, 50)]
+    assert peak[1] - peak[0] < (34 + 16) * n
 
 
 def _build(L, g, rank, K, B):
