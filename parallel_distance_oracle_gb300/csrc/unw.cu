@@ -165,7 +165,7 @@ __device__ void root_step_phase(const UnwDev &d, const uint32_t *roots, uint32_t
         if (MODE == 2) {  // the older labels are in already (rows_phase)
             if (lane == 0) {
                 UD_AT(row, r, d.n, 4) = 0;
-                bm_set(d.bm + (b & 1) * bm_words(d.n, d.words), d.words, r, idx, 0);
+                bm_set(d, d.bm + (b & 1) * bm_words(d.n, d.words), r, idx, 0);
             }
         } else
         for (uint32_t j = lane; j <= len; j += 32)

@@ -40,8 +40,8 @@ struct __align__(16) LastGroup {
 // word d.dbg and the access goes to a scratch slot instead (never a trap), so
 // a run reports where it would have left its buffer and keeps going.  Sites:
 // 0 CSR, 1 per-vertex state, 2 label pool, 3 BP rows, 4 dist_matrix,
-// 5 indicator rows, 6 tail / frontier / retry lists.  Release builds compile
-// the checks away.
+// 5 indicator rows, 6 tail / frontier / retry lists, 7 cover bitmaps.  Release
+// builds compile the checks away.
 #ifdef PADO_DEBUG_BOUNDS
 #define UD_AT(arr, i, lim, site) (::pado::dbg_ref((arr), (uint64_t)(i), (uint64_t)(lim), (site), d.dbg))
 #else
@@ -74,7 +74,7 @@ struct UnwDev {
     uint32_t *ind;        // n * words
     uint32_t *ind_stamp;  // batch + 1 when the row is valid
     uint8_t *dm;          // B * n
-    uint32_t *bm;         // cover bitmaps, two by batch parity (null: none), see BmShape
+    uint32_t *bm;         // cover bitmaps, two by batch parity (null: none), see BM_SLACKS
     uint32_t *status;
     unsigned long long *work;  // algorithmic-byte counters (profiling only)
 };
@@ -230,16 +230,18 @@ __host__ __device__ __forceinline__ bool bm_shape(uint32_t words)
 {
     return words >= 4 && words <= 128 && (words & (words - 1)) == 0;
 }
-__device__ __forceinline__ void bm_set(uint32_t *bm, uint32_t words, uint32_t h, uint32_t idx, uint32_t dist)
+__device__ __forceinline__ void bm_set(const UnwDev &d, uint32_t *bm, uint32_t h, uint32_t idx, uint32_t dist)
 {
-    uint32_t *row = bm + (uint64_t)h * BM_SLACKS * words + (idx >> 5);
-    for (uint32_t e = max(dist, 1u); e <= BM_SLACKS; ++e) atomicOr(row + (e - 1) * words, 1u << (idx & 31));
+    const uint64_t row = (uint64_t)h * BM_SLACKS * d.words + (idx >> 5);
+    for (uint32_t e = max(dist, 1u); e <= BM_SLACKS; ++e)
+        atomicOr(&UD_AT(bm, row + (e - 1) * d.words, bm_words(d.n, d.words), 7), 1u << (idx & 31));
 }
 // Clears the word that holds root idx (the others in it end with the same batch).
-__device__ __forceinline__ void bm_clear(uint32_t *bm, uint32_t words, uint32_t h, uint32_t idx, uint32_t dist)
+__device__ __forceinline__ void bm_clear(const UnwDev &d, uint32_t *bm, uint32_t h, uint32_t idx, uint32_t dist)
 {
-    uint32_t *row = bm + (uint64_t)h * BM_SLACKS * words + (idx >> 5);
-    for (uint32_t e = max(dist, 1u); e <= BM_SLACKS; ++e) row[(e - 1) * words] = 0u;
+    const uint64_t row = (uint64_t)h * BM_SLACKS * d.words + (idx >> 5);
+    for (uint32_t e = max(dist, 1u); e <= BM_SLACKS; ++e)
+        UD_AT(bm, row + (e - 1) * d.words, bm_words(d.n, d.words), 7) = 0u;
 }
 
 // dist_matrix rows and cover bitmaps of a batch's roots from their labels (fill)
@@ -261,9 +263,9 @@ __device__ void rows_phase(const UnwDev &d, const uint32_t *roots, uint32_t nroo
             const uint8_t dd = UD_AT(d.pool_dist, base + j, d.pool_cap, 2);
             UD_AT(row, h, d.n, 4) = fill ? dd : (uint8_t)U8_INF;
             if (fill)
-                bm_set(bm, d.words, h, idx, dd);
+                bm_set(d, bm, h, idx, dd);
             else
-                bm_clear(bm, d.words, h, idx, dd);
+                bm_clear(d, bm, h, idx, dd);
         }
     }
 }
@@ -510,9 +512,10 @@ __device__ __forceinline__ bool bp_covered_lanes(const UnwDev &d, uint32_t r, ui
     bool cov = false;
     unsigned long long open = 0, first = 0;  // roots with x in (iter, iter + 2]; those with x = iter + 1
     auto nibble = [](uint32_t m) { return (unsigned long long)(((m & 0x08040201u) * 0x01010101u) >> 24); };
-    const uint4 *row = reinterpret_cast<const uint4 *>(d.bpdp + (uint64_t)r * d.kp);
     for (uint32_t q = 0; q < d.kp / 16; ++q) {
-        const uint4 v = mine ? row[q] : make_uint4(~0u, ~0u, ~0u, ~0u);
+        const uint4 v = mine ? *reinterpret_cast<const uint4 *>(
+                                   &UD_AT(d.bpdp, (uint64_t)r * d.kp + q * 16, (uint64_t)d.n * d.kp, 3))
+                             : make_uint4(~0u, ~0u, ~0u, ~0u);
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -527,7 +530,7 @@ __device__ __forceinline__ bool bp_covered_lanes(const UnwDev &d, uint32_t r, ui
     need = __ballot_sync(FULL, open != 0);
     if (!need || __reduce_add_sync(FULL, (uint32_t)__popcll(open)) > BP_LANE_OPEN * __popc(need)) return cov;
     need = 0;
-    const ulonglong2 *rs = reinterpret_cast<const ulonglong2 *>(d.bps) + (uint64_t)r * d.K;
+    const ulonglong2 *sets = reinterpret_cast<const ulonglong2 *>(d.bps);
     while (open) {
         ulonglong2 a[2];
         int i[2];
@@ -535,7 +538,7 @@ __device__ __forceinline__ bool bp_covered_lanes(const UnwDev &d, uint32_t r, ui
         for (int u = 0; u < 2; ++u) {
             i[u] = open ? __ffsll(open) - 1 : -1;
             open &= open - 1;  // (0 stays 0)
-            a[u] = i[u] >= 0 ? rs[i[u]] : make_ulonglong2(0, 0);
+            a[u] = i[u] >= 0 ? UD_AT(sets, (uint64_t)r * d.K + i[u], (uint64_t)d.n * d.K, 3) : make_ulonglong2(0, 0);
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -839,7 +842,7 @@ __device__ void pull_heavy_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
             UD_AT(d.pool_hub, nbase + len + j, d.pool_cap, 2) = s + idx;
             UD_AT(d.pool_dist, nbase + len + j, d.pool_cap, 2) = (uint8_t)iter;
             if (is_root) UD_AT(bc.dm, (uint64_t)(t - s) * bc.dn + (s + idx - bc.base), (uint64_t)d.B * bc.dn, 4) = (uint8_t)iter;
-            if (MODE == 2 && is_root) bm_set(bc.bm, d.words, s + idx, t - s, iter);
+            if (MODE == 2 && is_root) bm_set(d, bc.bm, s + idx, t - s, iter);
             atomicMin(&hs.ctr[4], s + idx);
         }
         __syncthreads();
@@ -1130,8 +1133,10 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
                         v[u] = make_uint4(0, 0, 0, 0);
                         if (any && k < nst)
                             v[u] = *reinterpret_cast<const uint4 *>(
-                                bc.bm + ((uint64_t)wr.sh[k] * BM_SLACKS + min((uint32_t)wr.sd[k], BM_SLACKS) - 1u) * d.words +
-                                sub * 4);
+                                &UD_AT(bc.bm,
+                                       ((uint64_t)wr.sh[k] * BM_SLACKS + min((uint32_t)wr.sd[k], BM_SLACKS) - 1u) * d.words +
+                                           sub * 4,
+                                       bm_words(d.n, d.words), 7));
                     }
 #pragma unroll
                     for (int u = 0; u < BM_LOADS; ++u) {
@@ -1264,7 +1269,7 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
             UD_AT(d.pool_hub, base + len + j, d.pool_cap, 2) = s + idx;
             UD_AT(d.pool_dist, base + len + j, d.pool_cap, 2) = (uint8_t)iter;
             if (is_root) UD_AT(bc.dm, (uint64_t)(t - s) * bc.dn + (s + idx - bc.base), (uint64_t)d.B * bc.dn, 4) = (uint8_t)iter;
-            if (MODE == 2 && is_root) bm_set(bc.bm, d.words, s + idx, t - s, iter);
+            if (MODE == 2 && is_root) bm_set(d, bc.bm, s + idx, t - s, iter);
             mn = min(mn, s + idx);
         }
         mn = warp_min_u32(mn);
