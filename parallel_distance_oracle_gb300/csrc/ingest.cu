@@ -629,14 +629,12 @@ __global__ void __launch_bounds__(256) csr_check_kernel(const uint32_t *adj, con
     uint32_t f = 0;
 #pragma unroll 4
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < m; k += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t x = adj[k];
+        const uint32_t x = adj[k], y = adj[k ? k - 1 : 0];
+        // entry 0 has no predecessor, marked as a start or not (it is not when the
+        // first list ends beyond the entries)
+        const bool first = k == 0 || (starts[k >> 5] >> (k & 31) & 1u);
         if (x >= n) f |= 2u;
-        // entry 0 has no predecessor, marked as a start or not (it is not when
-        // the first list ends beyond the entries)
-        if (k && !(starts[k >> 5] >> (k & 31) & 1u)) {
-            const uint32_t y = adj[k - 1];
-            if (y < x || (y == x && w && w[k - 1] < w[k])) f |= 4u;
-        }
+        if (!first && (y < x || (y == x && w && w[k - 1] < w[k]))) f |= 4u;
     }
     if (f) atomicOr(flags, f);
 }
