@@ -66,8 +66,9 @@ void collect_locked()
 
 const char *work_slot_name(int i)
 {
-    static const char *names[WORK_SLOTS] = {"pull_kernel",      "mark_kernel",      "bp_sibling_kernel",
-                                            "bp_child_kernel",  "query_unw_kernel", "query_w_kernel",
+    // slots of one name (the bit-parallel steps share a launch) are added up
+    static const char *names[WORK_SLOTS] = {"pull_kernel",      "mark_kernel",      "bp_loop_kernel",
+                                            "bp_loop_kernel",   "query_unw_kernel", "query_w_kernel",
                                             "w_pull_kernel",    "w_mark_kernel",    "finalize_kernel",
                                             "pull.cycles.scan", "pull.cycles.bp",   "pull.cycles.dist",
                                             "pull.cycles.commit", "pull.cycles.heavy", "events.first_offers",
