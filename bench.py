@@ -749,12 +749,14 @@ def ingest_cpu(scale: int):
 
 
 # Algorithmic bytes of one launch of the ingest kernels, L = directed entries
-# (2 per edge), m = edges: the keys' build from the edge list and the keys each
-# radix pass reads and writes; the last of the entries' five passes writes the
-# adjacency (4 bytes) instead of keys.
-def ingest_kernel_bytes(kernel: str, m: int):
+# (2 per edge), m = edges, n = vertices: the keys' build from the edge list and
+# the keys each radix pass reads and writes, the mean over the entries' passes (8
+# bits each over a source and a destination rank); the last one writes the adjacency
+# (4 bytes) instead of keys.
+def ingest_kernel_bytes(kernel: str, m: int, n: int):
     L = 2 * m
-    return {"rs_scatter_kernel": (4 * 16 + 12) * L // 5, "rs_hist_kernel": 8 * L,
+    passes = -(-2 * max(1, (n - 1).bit_length()) // 8)
+    return {"rs_scatter_kernel": ((passes - 1) * 16 + 12) * L // passes, "rs_hist_kernel": 8 * L,
             "entry_key_kernel": 8 * m + 8 * m + 8 * L, "degree_kernel": 8 * m + 16 * m}.get(kernel)
 
 
@@ -860,7 +862,7 @@ def run_ingest(args):
         tot_ms = sum(x["ms"] for x in prof.values())
         top = max(prof, key=lambda k: prof[k]["ms"])
         tk = prof[top]
-        per = ingest_kernel_bytes(top, m)
+        per = ingest_kernel_bytes(top, m, n)
         avg_s = tk["ms"] / 1e3 / max(tk["launches"], 1)
         ach = per / avg_s / 1e9 if per else None
         roofline = {"kernel": top, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
