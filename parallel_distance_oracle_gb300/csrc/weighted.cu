@@ -74,8 +74,16 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr int WPULL_WARPS = 4, WLOOP_WARPS = 8;
 constexpr int32_t RMIN_EMPTY = INT_MAX;
 // Tails of at least this degree are worked on by the whole grid: their heads
-// in items of WITEM adjacency entries, then a block each (see WTails).
-constexpr uint32_t WHEAVY_DEG = 512, WITEM = 64;
+// in items of WITEM adjacency entries, then a block each (see WTails).  Where more
+// than WHEAVY_MAX vertices reach it the degree is doubled until no more do: with
+// thousands of tails as long as each other a warp each fills the grid, and the
+// second phase only costs.  n random vertices of average degree 800, ms of the
+// build with all of them split / none: n = 4,096 19.2 / 19.9 (B = 512) and
+// 27.2 / 23.1 (B = 128), 8,192 72.3 / 77.6 and 113 / 92, 12,000 172 / 163 and
+// 291 / 200; R-MAT s18/ef64 (12,616 vertices of 512 and more) 219 / 245, and 197 with
+// those of 1,024 split.
+constexpr uint32_t WHEAVY_DEG = 512, WHEAVY_MAX = 8192, WITEM = 64;
+constexpr uint32_t WHEAVY_CLASSES = 23;  // degrees from WHEAVY_DEG << k to twice that, below 2^32
 constexpr uint32_t WHEAVY_BIT = 0x80000000u;  // of tail_stamp (rounds stay far below 2^31)
 constexpr int32_t HMIN_EMPTY = 0x7f7f7f7f;  // above every distance; a byte fill writes it
 
@@ -170,10 +178,29 @@ __device__ __forceinline__ bool warp_reserve_w(const WDev &d, uint32_t v, uint32
     return true;
 }
 
-__global__ void __launch_bounds__(256) w_heavy_flag_kernel(const uint32_t *off, uint32_t n, uint32_t *tail_stamp)
+// Vertices per class of degree, added to classes[WHEAVY_CLASSES].
+__global__ void __launch_bounds__(256) w_heavy_count_kernel(const uint32_t *off, uint32_t n, uint32_t *classes)
 {
+    __shared__ uint32_t h[WHEAVY_CLASSES];
+    if (threadIdx.x < WHEAVY_CLASSES) h[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const uint32_t k = (off[v + 1] - off[v]) / WHEAVY_DEG;
+        if (k) atomicAdd(&h[31 - __clz(k)], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < WHEAVY_CLASSES && h[threadIdx.x]) atomicAdd(&classes[threadIdx.x], h[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(256) w_heavy_flag_kernel(const uint32_t *off, uint32_t n, const uint32_t *classes,
+                                                           uint32_t *tail_stamp)
+{
+    uint64_t least = WHEAVY_DEG;
+    uint32_t cnt = 0;
+    for (uint32_t k = 0; k < WHEAVY_CLASSES; ++k) cnt += classes[k];
+    for (uint32_t k = 0; cnt > WHEAVY_MAX; ++k, least *= 2) cnt -= classes[k];
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        tail_stamp[v] = off[v + 1] - off[v] >= WHEAVY_DEG ? WHEAVY_BIT : 0u;
+        tail_stamp[v] = off[v + 1] - off[v] >= least ? WHEAVY_BIT : 0u;
 }
 
 // A head h of round lid - 1 whose smallest accepted root is mn: its
@@ -1188,7 +1215,7 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     Arena zeros, ws;
     DBuf<unsigned long long> pool_top, log_top;
     DBuf<uint64_t> lab_off, last_pos0, last_pos1, rbase;
-    DBuf<uint32_t> lab_len, lab_cap, act_stamp0, act_stamp1, tail_stamp, vq_len, dt, status;
+    DBuf<uint32_t> lab_len, lab_cap, act_stamp0, act_stamp1, tail_stamp, vq_len, dt, status, hclasses;
     DBuf<uint32_t> last_cnt0, last_cnt1, last_min0, last_min1, rlen, front0, front1, tails, tails2, tails3, retry, news,
         news2, rr, heavy, counters;
     DBuf<int16_t> snap;
@@ -1199,6 +1226,7 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     for (DBuf<uint32_t> *x : {&lab_len, &lab_cap, &act_stamp0, &act_stamp1, &tail_stamp, &vq_len}) zeros.add(*x, n);
     zeros.add(dt, (uint64_t)n * B);
     zeros.add(status, 1);
+    zeros.add(hclasses, WHEAVY_CLASSES);
     zeros.add(ctl, 1);
     ws.add(last_pos0, n);
     ws.add(last_pos1, n);
@@ -1209,9 +1237,10 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     ws.add(rlen, B);
     ws.add(counters, 8);
     ws.add(snap, (uint64_t)B * B);
-    // at most m / WHEAVY_DEG vertices are heavy, with m / WITEM whole items and
-    // one partial each
-    const uint64_t hmax = std::min<uint64_t>(n, g.m / WHEAVY_DEG) + 1, imax = g.m / WITEM + hmax;
+    // at most m / WHEAVY_DEG vertices are heavy, and WHEAVY_MAX, with m / WITEM whole
+    // items and one partial each
+    const uint64_t hcan = std::min<uint64_t>(n, g.m / WHEAVY_DEG);
+    const uint64_t hmax = std::min<uint64_t>(hcan, WHEAVY_MAX) + 1, imax = g.m / WITEM + hmax;
     DBuf<int32_t> hmin;
     DBuf<uint32_t> ht[3];
     DBuf<uint2> hi[3];
@@ -1224,9 +1253,12 @@ LabelRun w_label(const DevGraph &g, uint32_t B, LabelStore &out, cudaStream_t s)
     ws.commit();
     zeros.mem.fill_bytes(0, s);
     hmin.fill_bytes(0x7f, s);
+    if (hcan > WHEAVY_MAX)  // else too few vertices for another degree
+        PADO_LAUNCH("w_heavy_count_kernel", s,
+                    w_heavy_count_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, hclasses.p));
     if (n)
         PADO_LAUNCH("w_heavy_flag_kernel", s,
-                    w_heavy_flag_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, tail_stamp.p));
+                    w_heavy_flag_kernel<<<grid_for(n, 256), 256, 0, s>>>(g.off.p, n, hclasses.p, tail_stamp.p));
     for (DBuf<int16_t> *t : {&buf, &vd})
         if (t->n)
             PADO_LAUNCH("w_fill_inf_kernel", s,
