@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256, 8) query_unw_kernel(IndexView v, uint32_t
     unsigned long long bytes = 0;
     for (uint32_t p = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * group; p < k; p += step) {
         if (ONE) {
-            const uint8_t d = query_unw_pair(v, pair_head(v, qa[p], qb[p], U8_INF), lane, qs[warp], bytes);
+            const uint8_t d = query_unw_pair<true>(v, pair_head(v, qa[p], qb[p], U8_INF), lane, qs[warp], bytes);
             if (lane == 0) out[p] = d;
             bytes += 9;
             continue;
@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256, 8) query_unw_kernel(IndexView v, uint32_t
         __syncwarp();
         uint8_t mine = 0;
         for (uint32_t j = 0; j < cnt; ++j) {
-            const uint8_t d = query_unw_pair(v, heads[warp][j], lane, qs[warp], bytes);
+            const uint8_t d = query_unw_pair<false>(v, heads[warp][j], lane, qs[warp], bytes);
             if ((uint32_t)lane == j) mine = d;
         }
         bytes += 9ull * cnt;  // endpoints, results
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) query_w_kernel(IndexView v, uint32_t k, u
     unsigned long long bytes = 0;
     for (uint32_t p = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * group; p < k; p += step) {
         if (ONE) {
-            const int16_t d = query_w_pair(v, pair_head(v, qa[p], qb[p], I16_INF), lane, qs[warp], bytes);
+            const int16_t d = query_w_pair<true>(v, pair_head(v, qa[p], qb[p], I16_INF), lane, qs[warp], bytes);
             if (lane == 0) out[p] = d;
             bytes += 10;
             continue;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256) query_w_kernel(IndexView v, uint32_t k, u
         __syncwarp();
         int16_t mine = 0;
         for (uint32_t j = 0; j < cnt; ++j) {
-            const int16_t d = query_w_pair(v, heads[warp][j], lane, qs[warp], bytes);
+            const int16_t d = query_w_pair<false>(v, heads[warp][j], lane, qs[warp], bytes);
             if ((uint32_t)lane == j) mine = d;
         }
         bytes += 10ull * cnt;  // endpoints, results

@@ -117,20 +117,34 @@ __device__ __forceinline__ uint32_t intersect_short(uint32_t av, uint32_t bv, co
 // The same for any two lists, la <= lb and not empty: the window holds (or
 // awaits) b's first entries.  32 hubs of a at a time are searched in the window
 // (7 steps in shared memory); whichever side ends at the lower hub moves on.
-template <typename D>
+// AHEAD, for batches that the chain of loads bounds: a's next hubs are read before the
+// search and the distances of a match are added a turn later, so that a turn
+// waits for one round trip instead of two (1,000 pairs, us: weighted complete
+// graph of 1,000 vertices, every hub shared, 24.7 -> 18.7; weighted random graph of
+// 6,000, 264 labels a vertex, 12.6 -> 10.5; 20,000 pairs of it 29.3 -> 26.0).  Where
+// the instructions bound it the plain form is as fast and needs fewer registers
+// (2M weighted pairs, s16: 338 us; 354 with both ahead).
+template <bool AHEAD, typename D>
 __device__ __forceinline__ uint32_t intersect_min(uint32_t *win, uint32_t av, const uint32_t *__restrict__ ha,
                                                   const D *__restrict__ da, uint32_t la,
                                                   const uint32_t *__restrict__ hb, const D *__restrict__ db,
                                                   uint32_t lb, uint32_t d, int lane)
 {
     window_ready();
-    uint32_t ia = 0, ib = 0;
+    uint32_t ia = 0, ib = 0, xa = d, xb = 0;
     for (;;) {
+        uint32_t an = 0;
+        if (AHEAD) an = ia + 32 + lane < la ? __ldg(ha + ia + 32 + lane) : 0xfffffffeu;
         uint32_t lo = 0;
 #pragma unroll
         for (uint32_t step = QWIN / 2; step > 0; step >>= 1)
             if (win[lo + step - 1] < av) lo += step;
-        if (ia + lane < la && win[lo] == av) d = min(d, (uint32_t)(int32_t)da[ia + lane] + (uint32_t)(int32_t)db[ib + lo]);
+        if (AHEAD) d = min(d, xa + xb);
+        if (ia + lane < la && win[lo] == av) {
+            xa = (uint32_t)(int32_t)da[ia + lane];
+            xb = (uint32_t)(int32_t)db[ib + lo];
+            if (!AHEAD) d = min(d, xa + xb);
+        }
         const uint32_t amax = __shfl_sync(FULL, av, (int)(min(la - ia, 32u) - 1));
         if (lb - ib > QWIN && amax > win[QWIN - 1]) {
             ib += QWIN;
@@ -139,14 +153,15 @@ __device__ __forceinline__ uint32_t intersect_min(uint32_t *win, uint32_t av, co
             window_ready();
         } else {
             ia += 32;
-            if (ia >= la) return d;
-            av = ia + lane < la ? __ldg(ha + ia + lane) : 0xfffffffeu;
+            if (ia >= la) return AHEAD ? min(d, xa + xb) : d;
+            av = AHEAD ? an : ia + lane < la ? __ldg(ha + ia + lane) : 0xfffffffeu;
         }
     }
 }
 
 // Distance of a pair on an unweighted index (every lane returns it).  `bytes`
 // accumulates the algorithmic bytes read (lane 0 only).
+template <bool AHEAD>
 __device__ __forceinline__ uint8_t query_unw_pair(const IndexView &v, const PairHead &h, int lane, QueryScratch &qs,
                                                   unsigned long long &bytes)
 {
@@ -185,13 +200,14 @@ __device__ __forceinline__ uint8_t query_unw_pair(const IndexView &v, const Pair
     }
     if (h.la)
         d = h.lb <= 32 ? intersect_short<uint8_t>(av, bv, v.dist8 + h.oa, v.dist8 + h.ob, d, lane)
-                       : intersect_min<uint8_t>(qs.win, av, v.hub + h.oa, v.dist8 + h.oa, h.la, v.hub + h.ob,
-                                                v.dist8 + h.ob, h.lb, d, lane);
+                       : intersect_min<AHEAD, uint8_t>(qs.win, av, v.hub + h.oa, v.dist8 + h.oa, h.la,
+                                                       v.hub + h.ob, v.dist8 + h.ob, h.lb, d, lane);
     d = __reduce_min_sync(FULL, d);
     return (uint8_t)(d >= (uint32_t)(U8_INF - 2) ? U8_INF : d);
 }
 
 // Same on a weighted index (int16 distances, I16_INF = unreachable).
+template <bool AHEAD>
 __device__ __forceinline__ int16_t query_w_pair(const IndexView &v, const PairHead &h, int lane, QueryScratch &qs,
                                                 unsigned long long &bytes)
 {
@@ -202,8 +218,8 @@ __device__ __forceinline__ int16_t query_w_pair(const IndexView &v, const PairHe
     uint32_t av, bv, d = (uint32_t)I16_INF;
     load_hubs(v, h, lane, qs.win, av, bv);
     d = h.lb <= 32 ? intersect_short<int16_t>(av, bv, v.dist16 + h.oa, v.dist16 + h.ob, d, lane)
-                   : intersect_min<int16_t>(qs.win, av, v.hub + h.oa, v.dist16 + h.oa, h.la, v.hub + h.ob,
-                                            v.dist16 + h.ob, h.lb, d, lane);
+                   : intersect_min<AHEAD, int16_t>(qs.win, av, v.hub + h.oa, v.dist16 + h.oa, h.la,
+                                                   v.hub + h.ob, v.dist16 + h.ob, h.lb, d, lane);
     d = __reduce_min_sync(FULL, d);
     return (int16_t)(d >= (uint32_t)(I16_INF - 2) ? I16_INF : d);
 }

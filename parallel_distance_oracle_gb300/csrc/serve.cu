@@ -78,10 +78,12 @@ __global__ void __launch_bounds__(256) serve_query_kernel(const ServeRun *__rest
         const ServeRun &run = runs[r];
         const uint64_t i = p - run.start;
         if (run.weighted) {
-            const int16_t d = query_w_pair(run.v, pair_head(run.v, qa[p], qb[p], I16_INF), lane, qs[threadIdx.x >> 5], bytes);
+            const int16_t d =
+                query_w_pair<true>(run.v, pair_head(run.v, qa[p], qb[p], I16_INF), lane, qs[threadIdx.x >> 5], bytes);
             if (lane == 0) reinterpret_cast<int16_t *>(out + run.out_off)[i] = d;
         } else {
-            const uint8_t d = query_unw_pair(run.v, pair_head(run.v, qa[p], qb[p], U8_INF), lane, qs[threadIdx.x >> 5], bytes);
+            const uint8_t d =
+                query_unw_pair<true>(run.v, pair_head(run.v, qa[p], qb[p], U8_INF), lane, qs[threadIdx.x >> 5], bytes);
             if (lane == 0) out[run.out_off + i] = d;
         }
     }
