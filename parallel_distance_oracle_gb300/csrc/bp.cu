@@ -52,9 +52,12 @@ constexpr int NB = 4;                // neighbours whose rows are loaded togethe
 // such vertex per block of the grid.  In a small graph a hub's neighbours, 32 at a time, are
 // a warp's chain that every level waits for; in a large one blocks for mid-degree
 // vertices would queue behind each other.  Judged by the degrees at doubling ids past the
-// grid (ids are ranks, most often by degree).  Against 2,048 for all (R-MAT, us of the
-// loop): s10/ef8 195 -> 137, s12/ef8 368 -> 174, s14/ef16 766 -> 358, s16/ef8 901 -> 608,
-// s18 and up the same.
+// grid (ids are ranks, most often by degree; in another order blocks get more of the
+// mid-degree vertices).  Against 2,048 for all (R-MAT, us of the loop): s10/ef8 195 ->
+// 137, s12/ef8 368 -> 174, s14/ef16 766 -> 358, s16/ef8 901 -> 608, s18 and up the same.
+// In random order, and against a launch per step with 2,048 (us of all BP work): s12/ef8
+// 650 -> 280, s14/ef16 1,140 -> 555, s16/ef8 1,330 -> 850; s18/ef16 by degree times
+// log-normal noise 3,250 -> 2,750.
 uint32_t heavy_degree(const HostGraph &hg, uint32_t grid)
 {
     uint32_t t = 64;

@@ -83,7 +83,8 @@ __global__ void __launch_bounds__(PULL_THREADS, 4) pull_kernel(UnwDev d, PullArg
 
 // ---------------------------------------------------------------------------
 // Persistent labeling loop: one cooperative launch runs batch after batch,
-// level after level, with ONE grid barrier per step:
+// level after level, with ONE grid barrier per step (two in a batch step with cover
+// bitmaps, whose rows are filled by several warps a root before the root's list moves):
 //   batch step (batch b at stamp L): each root r of b gets its self label
 //       (stamp L), fills dist_matrix row r - s from its labels and marks its
 //       own tails for L+1; the rows of batch b-1 are reset in the same step
@@ -167,9 +168,10 @@ __device__ void root_step_phase(const UnwDev &d, const uint32_t *roots, uint32_t
                 UD_AT(row, r, d.n, 4) = 0;
                 bm_set(d, d.bm + (b & 1) * bm_words(d.n, d.words), r, idx, 0);
             }
-        } else
-        for (uint32_t j = lane; j <= len; j += 32)
-            UD_AT(row, UD_AT(d.pool_hub, base + j, d.pool_cap, 2), d.n, 4) = UD_AT(d.pool_dist, base + j, d.pool_cap, 2);
+        } else {
+            for (uint32_t j = lane; j <= len; j += 32)
+                UD_AT(row, UD_AT(d.pool_hub, base + j, d.pool_cap, 2), d.n, 4) = UD_AT(d.pool_dist, base + j, d.pool_cap, 2);
+        }
         mark_tails(d, r, r, L + 1, bf.tails[nx], &c->tcnt[nx], bf.htails[nx], &c->hcnt[nx], lane, 0, 1, bytes);
     }
     if (d.work && lane == 0 && bytes) atomicAdd(&d.work[W_MARK], bytes);

@@ -1006,8 +1006,8 @@ __device__ void pull_light_tail(const UnwDev &d, const PullArgs &a, uint32_t t, 
         __syncwarp();
     }
     if (d.K > 1 && need2) {
-        // second stage for the unflagged survivors, two candidates per step,
-        // against t's whole row (lane i: roots i and i + 32), loaded only now
+        // second stage for the unflagged survivors, BP_GROUP at a time (or a lane
+        // each), against t's whole row (lane i: roots i and i + 32), loaded only now
         const uint8_t td0 = lane < (int)d.K ? UD_AT(d.bpd, (uint64_t)t * d.K + lane, (uint64_t)d.n * d.K, 3) : (uint8_t)U8_INF;
         const uint8_t td1 = lane + 32 < (int)d.K ? UD_AT(d.bpd, (uint64_t)t * d.K + lane + 32, (uint64_t)d.n * d.K, 3) : (uint8_t)U8_INF;
         const ulonglong2 ts0 =
